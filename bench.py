@@ -850,9 +850,9 @@ def main():
                          "aged pool from its checkpoint file (slots copied host-to-device), "
                          f"{max(args.steps, 10)} launches with a counter poll after each, outcomes copied back"),
                 "seconds": getattr(e2e_res, "e2e_split", None)},
-        # kernels per timed launch: the split step is three kernels per BD step plus the compaction's two;
+        # kernels per timed launch: the split step is three kernels per BD step plus one and the compaction's two;
         # the fused stepper is one kernel plus the compaction's two
-        "gpu_launches": ((3 * args.inner + 2) if launch["group"] == 66 else 3) * args.steps,
+        "gpu_launches": ((3 * args.inner + 3) if launch["group"] == 66 else 3) * args.steps,
         "clocks": ck,
     }
     if world == 1 and not args.no_surrogate and args.workload != "two-spheres":

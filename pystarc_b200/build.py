@@ -16,7 +16,8 @@ PKG = Path(__file__).resolve().parent
 ROOT = PKG.parent
 CSRC = PKG / "csrc"
 LIB = PKG / "libpystarc_b200.so"
-SOURCES = ["bd_api.cu", "bd_noalloc.cu", "bd_mlp.cu"]
+SOURCES = ["bd_api.cu", "bd_table_mixed.cu", "bd_table_mixed_torque.cu", "bd_table_fp64.cu", "bd_table_fp64_torque.cu",
+           "bd_noalloc.cu", "bd_mlp.cu"]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 FLAGS = ["-O3", "-std=c++17", *ARCH, "-lineinfo", "-Xcompiler", "-fPIC"]
 

@@ -8,11 +8,8 @@
 #include <string>
 #include <vector>
 
-#include "bd_kernels.cuh"
 #include "bd_nvtx.cuh"
-#include "bd_multi.cuh"
-#include "bd_surrogate.cuh"
-#include "bd_split.cuh"
+#include "bd_tables.cuh"
 #include "pystarc_b200.h"
 
 // surrogate MLP (bd_mlp.cu)
@@ -83,6 +80,8 @@ struct BdHandle {
   // split stepper (BD_GROUP_SPLIT): per-slot scratch of one step
   SplitBuf split_buf{};
   int split_cap = 0;
+  cudaStream_t side = nullptr;  // capture only: the force kernel that runs beside the other
+  cudaEvent_t fork = nullptr, join = nullptr;
   unsigned long long* sur_ctr_host_base = nullptr;
   // graphs: [cur][steps] cache
   cudaGraphExec_t graph[2] = {nullptr, nullptr};
@@ -607,44 +606,27 @@ cudaStream_t pick(BdHandle*, void* s) { return (cudaStream_t)s; }
 // ---------------------------------------------------------------------------
 // Kernel dispatch over (precision, group size, torque)
 // ---------------------------------------------------------------------------
-template <typename FT, int G, bool TQ>
-struct K {
-  static void* pose() { return (void*)&eval_pose_kernel<FT, G, TQ>; }
-  static void* atoms() { return (void*)&eval_atoms_kernel<FT, G, TQ>; }
-  static void* step() { return (void*)&step_kernel<FT, G, TQ>; }
-};
+const KernelTable& table_for(int prec, int torque) {
+  static const KernelTable tables[4] = {table_fp64(), table_fp64_torque(), table_mixed(), table_mixed_torque()};
+  return tables[(prec == BD_PREC_FP64 ? 0 : 2) + (torque == BD_TORQUE_CENTROID ? 1 : 0)];
+}
 
-template <typename FT, bool TQ>
-void* pick_g(int G, int which) {
+// which: 0 evaluation of poses, 1 evaluation with explicit atoms, 2 stepper
+void* kernel_for(int prec, int G, int torque, int which) {
+  const KernelTable& t = table_for(prec, torque);
   if (G == BD_GROUP_SPLIT) {
-    // the stepper's last phase sizes the slot pool; the parity kernels use a full-warp group
-    if (which == 2) return (void*)&split_end_kernel<FT, TQ>;
+    // the stepper has kernels of its own; the parity kernels use a full-warp group
+    if (which == 2) return t.split.mid;
     G = 32;
   }
   if (G == BD_GROUP_WARP || G == BD_GROUP_WARP_CAPPED) {
     // warp-cooperative stepper; the parity kernels use a full-warp group (same sweep code)
-    if (which == 2)
-      return G == BD_GROUP_WARP ? (void*)&step_kernel_warp<FT, TQ, 1> : (void*)&step_kernel_warp<FT, TQ, 2>;
+    if (which == 2) return G == BD_GROUP_WARP ? t.warp : t.warp_capped;
     G = 32;
   }
-  switch (G) {
-#define BD_CASE(g)                                                  \
-  case g:                                                           \
-    return which == 0 ? K<FT, g, TQ>::pose() : which == 1 ? K<FT, g, TQ>::atoms() : K<FT, g, TQ>::step();
-    BD_CASE(1)
-    BD_CASE(4)
-    BD_CASE(8)
-    BD_CASE(16)
-    BD_CASE(32)
-#undef BD_CASE
-  }
+  for (int i = 0; i < 5; ++i)
+    if (kGroups[i] == G) return which == 0 ? t.pose[i] : which == 1 ? t.atoms[i] : t.step[i];
   return nullptr;
-}
-
-void* kernel_for(int prec, int G, int torque, int which) {
-  const bool tq = torque == BD_TORQUE_CENTROID;
-  if (prec == BD_PREC_FP64) return tq ? pick_g<double, true>(G, which) : pick_g<double, false>(G, which);
-  return tq ? pick_g<float, true>(G, which) : pick_g<float, false>(G, which);
 }
 
 bool valid_group(int g) {
@@ -713,10 +695,12 @@ int launch_group_for(const BdHandle* h, int overlap) {
   if (h->launch_user) return h->group;
   const bool sweeps = h->S.born_rev || (overlap && !h->rec.empty());
   const int g = default_group(n_charged(h), sweeps);
-  if (g != BD_GROUP_WARP) return g;
-  // measured on the aged protein-ligand pool: the split step is fastest in mixed precision when
-  // there is a reverse-Born sweep; otherwise the fused kernel with registers capped at 128
-  return (h->S.born_rev && h->sp.precision == BD_PREC_MIXED) ? BD_GROUP_SPLIT : BD_GROUP_WARP_CAPPED;
+  // the split step is the faster one at every pool size measured (BD steps/s, fused kernel at 128
+  // registers -> split; protein + small ligand from the b-sphere): mixed 8,000 slots without
+  // reverse Born 127 -> 359 M, 600,000 with it 275 -> 365 M; FP64 150,000 171 -> 265 M, 600,000
+  // 209 -> 276 M; protein-protein FP64 6,000 slots 2.8 -> 19.9 M, 60,000 22.8 -> 37.8 M.  At
+  // 300,000 slots, mixed, without reverse Born they are level (882 and 879 M).
+  return g == BD_GROUP_WARP ? (int)BD_GROUP_SPLIT : g;
 }
 
 int launch_group(const BdHandle* h) { return launch_group_for(h, h->sp.overlap); }
@@ -733,6 +717,19 @@ int persistent_blocks(BdHandle* h, void* fn, int block, size_t smem = 0) {
   int per_sm = 0;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, block, smem) != cudaSuccess || per_sm < 1) per_sm = 1;
   return per_sm * h->n_sm;
+}
+
+// Resident blocks of h->block threads of a stepper: what the slot pool's size follows from.  The
+// split stepper's kernels have block sizes of their own; its pool stays that of a 128-register
+// kernel of h->block threads (with the shared memory of the fused kernel that was the default for
+// FP64 and without reverse Born), so that saved pools keep their capacity.
+int resident_blocks(BdHandle* h, int G, void* fn, size_t smem) {
+  if (G != BD_GROUP_SPLIT) return persistent_blocks(h, fn, h->block, smem);
+  int per_sm = 65536 / 128 / h->block, sm_bytes = 0;
+  cudaDeviceGetAttribute(&sm_bytes, cudaDevAttrMaxSharedMemoryPerMultiprocessor, h->device);
+  if (!h->launch_user) smem += h->sp.precision == BD_PREC_FP64 ? 16384 : h->S.born_rev ? 0 : 8192;
+  if (smem) per_sm = std::min<int>(per_sm, (int)((size_t)sm_bytes / (smem + 1024)));
+  return std::max(per_sm, 1) * h->n_sm;
 }
 
 // Dynamic shared memory of a stepper launch (block_shared_begin's layout): the
@@ -784,6 +781,9 @@ int bd_destroy(BdHandle* h) {
   free_tex(h->sys_tex);
   free_list(h->sys_allocs);
   free_list(h->sim_allocs);
+  if (h->fork) cudaEventDestroy(h->fork);
+  if (h->join) cudaEventDestroy(h->join);
+  if (h->side) cudaStreamDestroy(h->side);
   if (h->own) cudaStreamDestroy(h->own);
   delete h;
   return BD_OK;
@@ -1070,7 +1070,7 @@ int bd_get_launch(BdHandle* h, int* group, int* block, int* grid) {
   if (block) *block = h->block;
   if (grid) {
     void* fn = kernel_for(h->sp.precision, G, h->sp.torque_mode, 2);
-    *grid = fn ? persistent_blocks(h, fn, h->block, stepper_smem(h->S, h->P, fn)) : 0;
+    *grid = fn ? resident_blocks(h, G, fn, stepper_smem(h->S, h->P, fn)) : 0;
   }
   return BD_OK;
 }
@@ -1108,7 +1108,7 @@ int bd_sim_configure(BdHandle* h, const BdSimParams* p) {
   DevSim probe{};
   probe.stats = p->stats;
   const long long resident =
-      (long long)persistent_blocks(h, fn, h->block, stepper_smem(h->S, probe, fn)) * (h->block / lanes_per_traj(G));
+      (long long)resident_blocks(h, G, fn, stepper_smem(h->S, probe, fn)) * (h->block / lanes_per_traj(G));
   long long cap = p->slots > 0 ? p->slots : std::max<long long>(65536, 8 * resident);
   cap = std::min<long long>(cap, p->n_traj);
   const int C = (int)cap;
@@ -1287,33 +1287,26 @@ int ensure_surrogate_buffers(BdHandle* h) {
   return BD_OK;
 }
 
-extern "C++" {
-template <typename FT, bool TQ>
 int enqueue_surrogate_step(BdHandle* h, cudaStream_t s, int cur, int blocks) {
+  const KernelTable& t = table_for(h->sp.precision, h->sp.torque_mode);
   SlotBuf B = h->buf[cur];
   const int* live = h->d_live + cur;
   SurBuf U = h->sur_buf;
   zero_int_kernel<<<1, 1, 0, s>>>(U.n_rows);
-  sur_begin_kernel<FT, TQ><<<blocks, 256, 0, s>>>(h->S, h->P, B, live, U, h->sur_q);
-  CK(h, cudaGetLastError());
+  void* args[] = {&h->S, &h->P, &B, &live, &U, &h->sur_q};
+  CK(h, cudaLaunchKernel(t.sur_begin, dim3(blocks), dim3(256), args, 0, s));
   int rc = bd_internal_mlp_ensemble_rows(h->sur, h->sur_cap, U.n_rows, U.X, (float*)U.mean, (float*)U.spread, s);
   if (rc) return fail(h, rc, "surrogate: %s", bd_internal_mlp_error(h->sur));
-  sur_end_kernel<FT, TQ><<<blocks, 256, 0, s>>>(h->S, h->P, B, live, U, h->sur_q);
-  CK(h, cudaGetLastError());
+  CK(h, cudaLaunchKernel(t.sur_end, dim3(blocks), dim3(256), args, 0, s));
   return BD_OK;
 }
-}  // extern "C++"
 
 // K surrogate BD steps on buffer `cur`, then the compaction into the other buffer.
 int enqueue_surrogate_launch(BdHandle* h, int K, cudaStream_t s, int cur, int blocks) {
-  const bool tq = h->sp.torque_mode == BD_TORQUE_CENTROID, f64 = h->sp.precision == BD_PREC_FP64;
   // forces kept over rejected steps are per slot: the compaction between launches moves slots
   CK(h, cudaMemsetAsync(h->sur_buf.fresh, 0, (size_t)h->sur_cap, s));
   for (int k = 0; k < K; ++k) {
-    int rc = f64 ? (tq ? enqueue_surrogate_step<double, true>(h, s, cur, blocks)
-                       : enqueue_surrogate_step<double, false>(h, s, cur, blocks))
-                 : (tq ? enqueue_surrogate_step<float, true>(h, s, cur, blocks)
-                       : enqueue_surrogate_step<float, false>(h, s, cur, blocks));
+    int rc = enqueue_surrogate_step(h, s, cur, blocks);
     if (rc) return rc;
   }
   SlotBuf src = h->buf[cur], dst = h->buf[1 - cur];
@@ -1325,10 +1318,7 @@ int enqueue_surrogate_launch(BdHandle* h, int K, cudaStream_t s, int cur, int bl
 }
 
 int surrogate_blocks(BdHandle* h) {
-  const bool tq = h->sp.torque_mode == BD_TORQUE_CENTROID, f64 = h->sp.precision == BD_PREC_FP64;
-  void* fa = f64 ? (tq ? (void*)&sur_begin_kernel<double, true> : (void*)&sur_begin_kernel<double, false>)
-                 : (tq ? (void*)&sur_begin_kernel<float, true> : (void*)&sur_begin_kernel<float, false>);
-  return persistent_blocks(h, fa, 256);
+  return persistent_blocks(h, table_for(h->sp.precision, h->sp.torque_mode).sur_begin, 256);
 }
 
 // Scratch of the split stepper for the configured capacity (outside any capture).
@@ -1348,53 +1338,50 @@ int ensure_split_buffers(BdHandle* h) {
   U.rprev = (double*)q;
   if ((rc = dev_alloc(h, h->sim_allocs, &q, (size_t)C))) return rc;
   U.mode = (int8_t*)q;
-  if ((rc = dev_alloc(h, h->sim_allocs, &q, (size_t)C))) return rc;
-  U.fresh = (int8_t*)q;
   if ((rc = dev_alloc(h, h->sim_allocs, &q, (size_t)C * sizeof(int)))) return rc;
-  U.list = (int*)q;
-  if ((rc = dev_alloc(h, h->sim_allocs, &q, 2 * sizeof(int)))) return rc;
+  U.flist = (int*)q;
+  if ((rc = dev_alloc(h, h->sim_allocs, &q, (size_t)C * sizeof(int)))) return rc;
+  U.rlist = (int*)q;
+  if ((rc = dev_alloc(h, h->sim_allocs, &q, 8 * sizeof(int)))) return rc;
   U.cnt = (int*)q;
+  CK(h, cudaMemset(U.cnt, 0, 8 * sizeof(int)));
+  CK(h, cudaDeviceSynchronize());  // the legacy stream's memset, before any stream's launches
+  if (!h->side) CK(h, cudaStreamCreateWithFlags(&h->side, cudaStreamNonBlocking));
+  if (!h->fork) CK(h, cudaEventCreateWithFlags(&h->fork, cudaEventDisableTiming));
+  if (!h->join) CK(h, cudaEventCreateWithFlags(&h->join, cudaEventDisableTiming));
   h->split_cap = C;
   return BD_OK;
 }
 
-struct SplitKernels {
-  void *begin, *rev, *end;
-};
-
-extern "C++" {
-template <typename FT, bool TQ>
-SplitKernels split_kernels_t() {
-  return {(void*)&split_begin_kernel<FT, TQ>, (void*)&split_rev_kernel<FT, TQ>, (void*)&split_end_kernel<FT, TQ>};
-}
-}  // extern "C++"
-
-SplitKernels split_kernels(int prec, int torque) {
-  const bool tq = torque == BD_TORQUE_CENTROID;
-  if (prec == BD_PREC_FP64) return tq ? split_kernels_t<double, true>() : split_kernels_t<double, false>();
-  return tq ? split_kernels_t<float, true>() : split_kernels_t<float, false>();
-}
-
-// K split steps on buffer `cur` (three kernels each), then the compaction into the other buffer.
+// K split steps on buffer `cur`, then the compaction into the other buffer.  The two force
+// kernels of a step do not depend on each other: the sweep is captured on a branch of its own.
 int enqueue_split_launch(BdHandle* h, int K, cudaStream_t s, int cur) {
-  const SplitKernels kn = split_kernels(h->sp.precision, h->sp.torque_mode);
-  const size_t smem = stepper_smem(h->S, h->P, kn.end);
-  const int b_begin = persistent_blocks(h, kn.begin, 256), b_rev = persistent_blocks(h, kn.rev, 256),
-            b_end = persistent_blocks(h, kn.end, 256, smem);
+  const SplitKernels& kn = table_for(h->sp.precision, h->sp.torque_mode).split;
+  const size_t smem = stepper_smem(h->S, h->P, kn.mid);
+  stepper_smem(h->S, h->P, kn.last);
+  const int b_step = persistent_blocks(h, kn.mid, kStepBlock, smem), b_fwd = persistent_blocks(h, kn.fwd, 256),
+            b_rev = persistent_blocks(h, kn.rev, 256);
   SlotBuf src = h->buf[cur], dst = h->buf[1 - cur];
   const int* live = h->d_live + cur;
   SplitBuf U = h->split_buf;
-  unsigned long long* ctr = h->d_ctr;
-  // forces kept over rejected steps are per slot: the compaction between launches moves slots
-  CK(h, cudaMemsetAsync(U.fresh, 0, (size_t)h->split_cap, s));
-  for (int k = 0; k < K; ++k) {
-    CK(h, cudaMemsetAsync(U.cnt, 0, 2 * sizeof(int), s));
-    void* a_args[] = {&h->S, &h->P, &src, &live, &U};
-    CK(h, cudaLaunchKernel(kn.begin, dim3(b_begin), dim3(256), a_args, 0, s));
-    void* r_args[] = {&h->S, &src, &U, &ctr};
-    CK(h, cudaLaunchKernel(kn.rev, dim3(b_rev), dim3(256), r_args, 0, s));
-    void* e_args[] = {&h->S, &h->P, &src, &live, &U};
-    CK(h, cudaLaunchKernel(kn.end, dim3(b_end), dim3(256), e_args, smem, s));
+  OneTab T{h->S, h->P};
+  for (int k = 0; k <= K; ++k) {
+    int set = k & 1;
+    void* s_args[] = {&T, &src, &live, &U, &set};
+    if (k == K) {
+      CK(h, cudaLaunchKernel(kn.last, dim3(b_step), dim3(kStepBlock), s_args, smem, s));
+      break;
+    }
+    CK(h, cudaLaunchKernel(k == 0 ? kn.first : kn.mid, dim3(b_step), dim3(kStepBlock), s_args, k == 0 ? 0 : smem, s));
+    void* f_args[] = {&T, &src, &U, &set};
+    if (h->S.born_rev) {
+      CK(h, cudaEventRecord(h->fork, s));
+      CK(h, cudaStreamWaitEvent(h->side, h->fork, 0));
+      CK(h, cudaLaunchKernel(kn.rev, dim3(b_rev), dim3(256), f_args, 0, h->side));
+      CK(h, cudaEventRecord(h->join, h->side));
+    }
+    CK(h, cudaLaunchKernel(kn.fwd, dim3(b_fwd), dim3(256), f_args, 0, s));
+    if (h->S.born_rev) CK(h, cudaStreamWaitEvent(s, h->join, 0));
   }
   compact_kernel<<<h->n_sm * 4, 256, 0, s>>>(src, dst, live, h->d_ctr);
   CK(h, cudaGetLastError());
@@ -1415,7 +1402,7 @@ int build_graphs(BdHandle* h, int K) {
     }
   void* fn = kernel_for(h->sp.precision, G, h->sp.torque_mode, 2);
   const size_t smem = stepper_smem(h->S, h->P, fn);
-  const int blocks = persistent_blocks(h, fn, h->block, smem);
+  const int blocks = resident_blocks(h, G, fn, smem);
   const int sblocks = h->sur ? surrogate_blocks(h) : 0;
   if (h->sur) {
     int rc = ensure_surrogate_buffers(h);
@@ -1841,11 +1828,7 @@ int malloc_multi(BdMulti* m, void** p, size_t bytes) {
   return BD_OK;
 }
 
-void* multi_kernel(int prec, int torque) {
-  const bool tq = torque == BD_TORQUE_CENTROID;
-  if (prec == BD_PREC_FP64) return tq ? (void*)&step_kernel_multi<double, true> : (void*)&step_kernel_multi<double, false>;
-  return tq ? (void*)&step_kernel_multi<float, true> : (void*)&step_kernel_multi<float, false>;
-}
+void* multi_kernel(int prec, int torque) { return table_for(prec, torque).multi; }
 
 int multi_graphs(BdMulti* m, int K) {
   if (m->graph_K == K) return BD_OK;

@@ -803,7 +803,7 @@ __device__ __forceinline__ void ov_cell_dist(const OvGeom& G, int i, int j, int 
 // One thread per cell.  Pass 1 (list == NULL): class (0 empty, 1 full, 2 mixed) and the
 // number of listed atoms.  Pass 2: the atoms of each mixed cell, in bin order, at the offset
 // held in its cell word.
-__global__ void ov_cells_kernel(const double4* __restrict__ rec, const int* __restrict__ bin_start,
+static __global__ void ov_cells_kernel(const double4* __restrict__ rec, const int* __restrict__ bin_start,
                                 const int* __restrict__ bin_atoms, OvGeom G, uint8_t* __restrict__ cls,
                                 int* __restrict__ cnt, const uint32_t* __restrict__ word, int* __restrict__ list) {
   const long n_cells = (long)G.n[0] * G.n[1] * G.n[2];
@@ -846,7 +846,7 @@ __global__ void ov_cells_kernel(const double4* __restrict__ rec, const int* __re
   }
 }
 
-__global__ void eval_overlap_kernel(DevSystem S, long long n, const double* __restrict__ cen, int8_t* __restrict__ out) {
+static __global__ void eval_overlap_kernel(DevSystem S, long long n, const double* __restrict__ cen, int8_t* __restrict__ out) {
   for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
     const double c[3] = {cen[3 * t], cen[3 * t + 1], cen[3 * t + 2]};
     out[t] = (int8_t)overlap_any<1>(S, c, 0, 1u);
@@ -1201,7 +1201,7 @@ __device__ __forceinline__ int group_fetch(unsigned long long* p, int lane, unsi
 
 // Window copy of a grid (DevGrid::win): entry n holds nodes n .. n + 4/ch - 1 of
 // node n's z row, all `ch` channels of each, zero past the end of the row.
-__global__ void window_kernel(const float* __restrict__ d, float4* __restrict__ w, long n_nodes, int nz, int ch) {
+static __global__ void window_kernel(const float* __restrict__ d, float4* __restrict__ w, long n_nodes, int nz, int ch) {
   for (long n = blockIdx.x * (long)blockDim.x + threadIdx.x; n < n_nodes; n += (long)gridDim.x * blockDim.x) {
     const int z = (int)(n % nz);
     float v[4];
@@ -1216,7 +1216,7 @@ __global__ void window_kernel(const float* __restrict__ d, float4* __restrict__ 
 
 // Cube copy of a one-channel grid (DevGrid::cube): entry n = (x, y, z) holds the 2x2x2 block
 // v(x + i, y + j, z + k) at 4i + 2j + k, zero past the grid's faces.
-__global__ void cube_kernel(const float* __restrict__ d, float* __restrict__ cube, int nx, int ny, int nz) {
+static __global__ void cube_kernel(const float* __restrict__ d, float* __restrict__ cube, int nx, int ny, int nz) {
   const long n_nodes = (long)nx * ny * nz;
   for (long n = blockIdx.x * (long)blockDim.x + threadIdx.x; n < n_nodes; n += (long)gridDim.x * blockDim.x) {
     const int z = (int)(n % nz), y = (int)((n / nz) % ny), x = (int)(n / ((long)ny * nz));
@@ -1238,7 +1238,7 @@ __global__ void cube_kernel(const float* __restrict__ d, float* __restrict__ cub
 // The xy records of a one-channel grid (DevGrid::xy): per node, for each cell half in x and y,
 // the extra x plane's four nodes and the extra y row's four nodes of the stencil (nodes off the
 // grid read as 0; stencils never reach them, every stencil position lies in the margin box).
-__global__ void xy_kernel(const float* __restrict__ d, float* __restrict__ xy, int nx, int ny, int nz) {
+static __global__ void xy_kernel(const float* __restrict__ d, float* __restrict__ xy, int nx, int ny, int nz) {
   const long n_nodes = (long)nx * ny * nz;
   auto at = [&](int x, int y, int z) -> float {
     return (x >= 0 && x < nx && y >= 0 && y < ny && z >= 0 && z < nz) ? d[((long)x * ny + y) * nz + z] : 0.f;
@@ -1266,7 +1266,7 @@ __global__ void xy_kernel(const float* __restrict__ d, float* __restrict__ xy, i
 }
 
 // z-edge records of a one-channel grid (DevGrid::ztex); nodes off the grid read as 0.
-__global__ void zedge_kernel(const float* __restrict__ d, float4* __restrict__ out, int nx, int ny, int nz) {
+static __global__ void zedge_kernel(const float* __restrict__ d, float4* __restrict__ out, int nx, int ny, int nz) {
   const long n_nodes = (long)nx * ny * nz;
   auto at = [&](int x, int y, int z) -> float {
     return (x >= 0 && x < nx && y >= 0 && y < ny && z >= 0 && z < nz) ? d[((long)x * ny + y) * nz + z] : 0.f;
@@ -1289,7 +1289,7 @@ __global__ void hi_diffusion_kernel(DevSim P, int n, const double* __restrict__ 
 }
 
 // Fill `n_slots` slots with the first trajectories of the pending pool.
-__global__ void init_slots_kernel(DevSim P, SlotBuf B, int n_slots) {
+static __global__ void init_slots_kernel(DevSim P, SlotBuf B, int n_slots) {
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= n_slots) return;
   Traj tr;
@@ -1536,7 +1536,7 @@ __device__ __forceinline__ void flush_tally(const DevSim& P, Tally tl, bool owne
 
 // Move live slots of `src` (status RUNNING) densely into `dst`; the order is
 // irrelevant because every draw is keyed by trajectory id and step.
-__global__ void compact_kernel(SlotBuf src, SlotBuf dst, const int* __restrict__ n_live_src,
+static __global__ void compact_kernel(SlotBuf src, SlotBuf dst, const int* __restrict__ n_live_src,
                                unsigned long long* ctr) {
   const int n = *n_live_src;
   for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < n; s += gridDim.x * blockDim.x) {
@@ -1556,7 +1556,7 @@ __global__ void compact_kernel(SlotBuf src, SlotBuf dst, const int* __restrict__
 }
 
 // Publish the compacted count and reset the cursors for the next launch.
-__global__ void finish_compact_kernel(int* n_live_dst, unsigned long long* ctr) {
+static __global__ void finish_compact_kernel(int* n_live_dst, unsigned long long* ctr) {
   *n_live_dst = (int)ctr[C_LIVE_NEXT];
   ctr[C_LIVE_NEXT] = 0;
   ctr[C_SLOT_CURSOR] = 0;

@@ -99,7 +99,7 @@ __device__ __forceinline__ void multi_refill(const MultiTab& T, Traj& tr, int& s
   }
 }
 
-__global__ void init_slots_multi_kernel(MultiTab T, SlotBuf B, int n_slots) {
+static __global__ void init_slots_multi_kernel(MultiTab T, SlotBuf B, int n_slots) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n_slots) return;
   const int s = sys_of(T, i);

@@ -1,28 +1,32 @@
-// Split stepper: one BD step as three kernels instead of one fused persistent kernel.
+// Split stepper: one BD step as a scalar kernel over the slots and two force kernels over lists
+// of poses, instead of one fused persistent kernel.
 //
-//   split_begin_kernel  reaction test and escape/return (step_begin), the forces on the
-//                       ligand atoms (grid, far-field, contact), and the list of poses whose
-//                       receptor atoms can reach the ligand Born grid
-//   split_rev_kernel    Born direction 2 of the listed poses, one warp per pose
-//   split_end_kernel    the rest of the step (step_move, overlap test, step_end, statistics)
-//                       and the refill of ended trajectories from the pending pool
+//   split_step_kernel  one lane per slot: the end of the previous step (step_move, overlap test,
+//                      step_end, statistics, refill of ended trajectories from the pending pool)
+//                      and the beginning of the next one (reaction test, escape/return), which
+//                      lists the poses whose forces are needed
+//   split_fwd_kernel   forces on the ligand atoms (grid, far-field, contact) of the listed poses
+//   split_rev_kernel   Born direction 2 of the listed poses that reach the ligand Born grid
 //
-// Near contact Born direction 2 is most of a step's work, and it is bound by the latency of
-// its grid gathers.  In the fused kernel it shares the per-trajectory state's registers
-// (128 per thread: 16 warps per SM); here it runs in a kernel capped at 64 registers, so
-// twice as many warps hide the gather latency.  Candidates (receptor atoms inside the
-// ligand's Born box, in the ligand frame) go to a per-warp buffer in shared memory and are
-// drained in whole groups of 32, entry i by lane i mod 32, in the order of the fused
-// kernel's ring: every lane sums the same terms in the same order, so the forces, and so
-// the trajectories, are those of the fused stepper.  The same keyed Philox stream drives
-// both (gpu_batch_simulator.py:783-1254 is the step being split).
+// The force kernels take one pose per warp from their list, so the warps of a pool share its
+// poses evenly whatever its size: with the forces inside the scalar kernel, a warp evaluated its
+// own 32 trajectories one after another, and a pool of 8,000 kept 250 warps busy on 148 SMs
+// (protein + small ligand, 8,000 slots: 74 us of forces in that kernel; 6,000 slots of a
+// 1,401-atom ligand: 1,140 us).  Each kernel also gets the registers that suit it: the scalar
+// step and the forward stencils 128, the latency-bound sweep of direction 2 64 (twice the warps).
+// Candidates of the sweep (receptor atoms inside the ligand's Born box, in the ligand frame) go
+// to a per-warp buffer in shared memory and are drained in whole groups of 32, entry i by lane i
+// mod 32, in the order of the fused kernel's ring: every lane sums the same terms in the same
+// order, so the forces, and so the trajectories, are those of the fused stepper.  The same keyed
+// Philox stream drives both (gpu_batch_simulator.py:783-1254 is the step being split).
 #pragma once
 
 #include "bd_kernels.cuh"
 
 namespace bd {
 
-constexpr int kSplitBuf = 128;  // candidate entries per warp (whole groups of 32 are drained)
+constexpr int kSplitBuf = 128;   // candidate entries per warp (whole groups of 32 are drained)
+constexpr int kStepBlock = 128;  // threads of a scalar-kernel block
 
 // Per-slot scratch of one BD step.
 struct SplitBuf {
@@ -32,99 +36,214 @@ struct SplitBuf {
   double* rprev;   // cap: |c| at the end of the previous step (statistics)
   int8_t* mode;    // 0: no step; 1: F, T to be used as they are; 2: reused (complete);
                    // 3: F, T plus the Born direction 2 sums in rv
-  int8_t* fresh;   // F, T hold the complete forces of the slot's current pose
-  int* list;       // slots listed for the sweep this step
-  int* cnt;        // [0] list length, [1] sweep cursor (both cleared before every step)
+  int* flist;      // slots listed for split_fwd_kernel this step
+  int* rlist;      // slots listed for split_rev_kernel this step
+  int* cnt;        // two sets of {flist length, rlist length, their cursors}, used by steps in
+                   // turn: a step's scalar kernel fills one set and clears the other
 };
 
-// Forces on the ligand atoms of every lane with `need`, the warp sweeping one pose at a time.
-template <typename FT, bool TORQUE>
-__device__ __forceinline__ void warp_forces_ligand(const DevSystem& S, const double c[3], const double R[9],
-                                                   bool need, double F[3], double T[3], int lane, Counts& cnt,
-                                                   const RecView& v) {
-  const unsigned FULL = 0xffffffffu;
-  unsigned m = __ballot_sync(FULL, need);
-  while (m) {
-    const int j = __ffs(m) - 1;
-    m &= m - 1;
-    double cj[3], Rj[9];
-#pragma unroll
-    for (int k = 0; k < 3; ++k) cj[k] = __shfl_sync(FULL, c[k], j);
-#pragma unroll
-    for (int k = 0; k < 9; ++k) Rj[k] = __shfl_sync(FULL, R[k], j);
-    double f[3], t[3], e;
-    group_forces<FT, 32, TORQUE, false, PosFromPose, false>(S, cj, Rj, lane, FULL, PosFromPose{Rj, cj}, f, t, e,
-                                                           cnt, v);
-    if (lane == j) {
-#pragma unroll
-      for (int k = 0; k < 3; ++k) {
-        F[k] = f[k];
-        T[k] = t[k];
-      }
-    }
+// One receptor-ligand system for all slots.
+struct OneTab {
+  DevSystem S;
+  DevSim P;
+  __device__ __forceinline__ const DevSystem& sys(int) const { return S; }
+  __device__ __forceinline__ const DevSim& sim(int) const { return P; }
+  __device__ __forceinline__ int locate(int&) const { return 0; }  // trajectory id -> system, local id
+  __device__ __forceinline__ int global_id(int, int id) const { return id; }
+  __device__ __forceinline__ void refill(Traj& tr, int&, bool& dead, int lane) const { warp_refill(P, tr, dead, lane); }
+  __device__ __forceinline__ bool overlap(int, const double cn[3], bool need, int lane, const RecView& v) const {
+    return warp_overlap(S, cn, need, lane, v);
   }
+};
+
+// Append the lanes with `want` to a list whose length is *len: one atomic per warp.
+__device__ __forceinline__ void warp_append(int* list, int* len, bool want, int value, int lane) {
+  const unsigned m = __ballot_sync(0xffffffffu, want);
+  if (!m) return;
+  int at = 0;
+  if (lane == __ffs(m) - 1) at = atomicAdd(len, __popc(m));
+  at = __shfl_sync(0xffffffffu, at, __ffs(m) - 1);
+  if (want) list[at + __popc(m & ((1u << lane) - 1u))] = value;
 }
 
-template <typename FT, bool TORQUE>
-__global__ void __launch_bounds__(256, 2) split_begin_kernel(DevSystem S, DevSim P, SlotBuf B,
-                                                             const int* __restrict__ n_live, SplitBuf U) {
-  const unsigned FULL = 0xffffffffu;
-  const int lane = threadIdx.x & 31;
-  const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, n_warps = (gridDim.x * blockDim.x) >> 5;
+// END: finish the step begun by the previous launch of this kernel; BEGIN: begin the next one.
+// Warp w of block b takes the slots of chunk w * gridDim.x + b, so a small pool spreads over the SMs.
+template <typename FT, bool TORQUE, bool END, bool BEGIN, class TAB>
+__global__ void __launch_bounds__(kStepBlock, 4) split_step_kernel(const __grid_constant__ TAB T, SlotBuf B,
+                                                                   const int* __restrict__ n_live, SplitBuf U,
+                                                                   int set) {
   const int live = *n_live;
+  if (blockIdx.x == 0 && threadIdx.x < 4) {
+    U.cnt[4 * (1 - set) + threadIdx.x] = 0;
+    if (!BEGIN) U.cnt[4 * set + threadIdx.x] = 0;
+  }
+  if ((long long)blockIdx.x * 32 >= live) return;  // no slots for this block
+  const DevSim& P0 = T.sim(0);
+  const BlockShared sh = END ? block_shared_begin(T.sys(0), P0) : BlockShared{RecView{nullptr, nullptr}, nullptr};
+  const int lane = threadIdx.x & 31;
+  const int n_warps = (gridDim.x * blockDim.x) >> 5;
   Tally tl{};
-  for (int base = warp * 32; base < live; base += n_warps * 32) {
-    const int slot = base + lane;
+  for (long long base = 32ll * ((threadIdx.x >> 5) * gridDim.x + blockIdx.x); base < live; base += 32ll * n_warps) {
+    const int slot = (int)base + lane;
     const bool own = slot < live;
     Traj tr{};
     tr.status = ST_EMPTY;
-    if (own) load_slot(B, slot, tr);
-    const bool run = own && tr.status == ST_RUNNING;
-    const uint32_t s = (uint32_t)tr.steps;
-    if (run && P.stats) U.rprev[slot] = norm3(tr.c[0], tr.c[1], tr.c[2]);
-    double R[9] = {1, 0, 0, 0, 1, 0, 0, 0, 1}, r = 0;
-    int st = ST_EMPTY;
-    const int rets0 = tr.rets;
-    if (run) {
-      st = step_begin(S, P, traj_key(P, tr.id), s, tr, R, r, tl);
-      if (P.stats && st == ST_REACTED) stats_encounter(P, tr, s, false);
-    }
-    const bool need = run && st == ST_RUNNING;
-    // a step rejected by the overlap test left the pose unchanged: its forces are reused
-    const bool reuse = need && tr.rets == rets0 && U.fresh[slot];
-    const bool eval = need && !reuse;
-    double F[3] = {0, 0, 0}, T[3] = {0, 0, 0};
-    warp_forces_ligand<FT, TORQUE>(S, tr.c, R, eval, F, T, lane, tl.cnt, RecView{nullptr, nullptr});
-    const bool rev = eval && S.born_rev && r - S.rec_max_r < S.lig_born_rho;
-    const unsigned rm = __ballot_sync(FULL, rev);
-    if (rm) {
-      int at = 0;
-      if (lane == __ffs(rm) - 1) at = atomicAdd(U.cnt, __popc(rm));
-      at = __shfl_sync(FULL, at, __ffs(rm) - 1);
-      if (rev) U.list[at + __popc(rm & ((1u << lane) - 1u))] = slot;
-    }
-    if (run && st != ST_RUNNING) {
-      tr.status = st;
-      P.out_status[tr.id] = (int8_t)st;
-      P.out_steps[tr.id] = tr.steps;
-      P.out_returns[tr.id] = tr.rets;
-      tl.reacted += st == ST_REACTED;
-      tl.escaped += st == ST_ESCAPED;
-      tl.maxsteps += st == ST_MAXSTEPS;
-    }
+    int k = 0;
     if (own) {
-      store_slot(B, slot, tr);
-      if (eval) {
+      load_slot(B, slot, tr);
+      k = T.locate(tr.id);
+    }
+    bool keep = false;  // F, T in the scratch are the forces at the slot's pose
+    if (END) {
+      const DevSystem& S = T.sys(k);
+      const DevSim& P = T.sim(k);
+      const int mode = own ? (int)U.mode[slot] : 0;
+      const bool need = mode != 0;
+      double R[9] = {1, 0, 0, 0, 1, 0, 0, 0, 1}, r = 0;
+      double F[3] = {0, 0, 0}, Tq[3] = {0, 0, 0};
+      if (need) {
+        quat_to_rot(tr.q, R);
+        r = norm3(tr.c[0], tr.c[1], tr.c[2]);
 #pragma unroll
-        for (int k = 0; k < 3; ++k) {
-          U.F[3 * slot + k] = F[k];
-          U.T[3 * slot + k] = T[k];
+        for (int i = 0; i < 3; ++i) {
+          F[i] = U.F[3 * slot + i];
+          Tq[i] = U.T[3 * slot + i];
+        }
+        if (mode == 3) {
+          // the reverse-Born force on the receptor, rotated to the lab frame, acts on the ligand
+          // with the opposite sign
+          const double* rv = U.rv + 6 * slot;
+#pragma unroll
+          for (int i = 0; i < 3; ++i) F[i] = F[i] - (R[3 * i] * rv[0] + R[3 * i + 1] * rv[1] + R[3 * i + 2] * rv[2]);
+          if (TORQUE) {
+#pragma unroll
+            for (int i = 0; i < 3; ++i)
+              Tq[i] = Tq[i] - (R[3 * i] * rv[3] + R[3 * i + 1] * rv[4] + R[3 * i + 2] * rv[5]);
+          }
         }
       }
-      U.mode[slot] = (int8_t)(need ? (reuse ? 2 : rev ? 3 : 1) : 0);
+      const Keyed key = traj_key(P, tr.id);
+      const uint32_t s = (uint32_t)tr.steps;
+      double cn[3] = {0, 0, 0}, qn[4] = {1, 0, 0, 0}, dt = 0;
+      bool ok = true;
+      if (need) ok = step_move<FT>(S, P, key, s, tr, R, r, F, Tq, cn, qn, dt);
+      int st = tr.status;
+      if (need && !ok) {
+        tl.nonfinite += 1;
+        st = ST_ERROR;
+      }
+      const bool ovl = T.overlap(k, cn, need && ok && P.overlap, lane, sh.v);
+      if (need && ok) {
+        const double c0[3] = {tr.c[0], tr.c[1], tr.c[2]};
+        st = step_end(S, P, key, s, tr, R, cn, qn, !ovl, dt, tl);
+        if (P.stats) {
+          stats_step(S, P, tr, s, U.rprev[slot], dt, c0, R, sh.stats);
+          trace_step(P, tr, s, F, dt);
+          if (st == ST_REACTED) stats_encounter(P, tr, s, true);
+        }
+      }
+      if (need && st != ST_RUNNING) {
+        tr.status = st;
+        P.out_status[tr.id] = (int8_t)st;
+        P.out_steps[tr.id] = tr.steps;
+        P.out_returns[tr.id] = tr.rets;
+        tl.reacted += st == ST_REACTED;
+        tl.escaped += st == ST_ESCAPED;
+        tl.maxsteps += st == ST_MAXSTEPS;
+      }
+      bool dead = !own;
+      T.refill(tr, k, dead, lane);
+      // rejected and still running: the next step starts from the same pose with these forces
+      keep = need && ok && ovl && st == ST_RUNNING;
+      if (BEGIN && keep && mode != 2) {
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+          U.F[3 * slot + i] = F[i];
+          U.T[3 * slot + i] = Tq[i];
+        }
+      }
+    }
+    if (BEGIN) {
+      const DevSystem& S = T.sys(k);
+      const DevSim& P = T.sim(k);
+      const bool run = own && tr.status == ST_RUNNING;
+      const uint32_t s = (uint32_t)tr.steps;
+      if (run && P.stats) U.rprev[slot] = norm3(tr.c[0], tr.c[1], tr.c[2]);
+      double R[9], r = 0;
+      int st = ST_EMPTY;
+      const int rets0 = tr.rets;
+      if (run) {
+        st = step_begin(S, P, traj_key(P, tr.id), s, tr, R, r, tl);
+        if (P.stats && st == ST_REACTED) stats_encounter(P, tr, s, false);
+      }
+      const bool need = run && st == ST_RUNNING;
+      const bool reuse = need && keep && tr.rets == rets0;
+      const bool eval = need && !reuse;
+      const bool rev = eval && S.born_rev && r - S.rec_max_r < S.lig_born_rho;
+      warp_append(U.flist, U.cnt + 4 * set, eval, slot, lane);
+      warp_append(U.rlist, U.cnt + 4 * set + 1, rev, slot, lane);
+      if (run && st != ST_RUNNING) {
+        tr.status = st;
+        P.out_status[tr.id] = (int8_t)st;
+        P.out_steps[tr.id] = tr.steps;
+        P.out_returns[tr.id] = tr.rets;
+        tl.reacted += st == ST_REACTED;
+        tl.escaped += st == ST_ESCAPED;
+        tl.maxsteps += st == ST_MAXSTEPS;
+      }
+      if (own) U.mode[slot] = (int8_t)(need ? (reuse ? 2 : rev ? 3 : 1) : 0);
+    }
+    if (own) {
+      tr.id = T.global_id(k, tr.id);
+      store_slot(B, slot, tr);
     }
   }
-  flush_tally(P, tl, true);
+  flush_tally(P0, tl, true);
+  if (END) stats_block_end(P0, sh.stats);
+}
+
+// The next item of a warp after its first: the cursor counts the items taken beyond one per warp.
+__device__ __forceinline__ int next_item(int* cursor, int n_warps, int lane) {
+  int j = 0;
+  if (lane == 0) j = n_warps + atomicAdd(cursor, 1);
+  return __shfl_sync(0xffffffffu, j, 0);
+}
+
+// Forces on the ligand atoms of the listed poses, one warp per pose.
+template <typename FT, bool TORQUE, class TAB>
+__global__ void __launch_bounds__(256, 2) split_fwd_kernel(const __grid_constant__ TAB T, SlotBuf B, SplitBuf U,
+                                                           int set) {
+  const unsigned FULL = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  const int n = U.cnt[4 * set], n_warps = (gridDim.x * blockDim.x) >> 5;
+  Counts cnt{0, 0, 0};
+  for (int j = (threadIdx.x >> 5) * gridDim.x + blockIdx.x; j < n;
+       j = next_item(U.cnt + 4 * set + 2, n_warps, lane)) {
+    const int slot = U.flist[j];
+    int id = B.traj[slot];
+    const DevSystem& S = T.sys(T.locate(id));
+    const double q[4] = {B.q[slot], B.q[B.cap + slot], B.q[2 * B.cap + slot], B.q[3 * B.cap + slot]};
+    const double c[3] = {B.c[slot], B.c[B.cap + slot], B.c[2 * B.cap + slot]};
+    double R[9], f[3], t[3], e;
+    quat_to_rot(q, R);
+    // the rotation as the fused stepper has it, a set of values: without this the compiler may fuse
+    // its arithmetic with the atoms' and round the positions otherwise
+#pragma unroll
+    for (int i = 0; i < 9; ++i) asm volatile("" : "+d"(R[i]));
+    group_forces<FT, 32, TORQUE, false, PosFromPose, false>(S, c, R, lane, FULL, PosFromPose{R, c}, f, t, e, cnt,
+                                                           RecView{nullptr, nullptr});
+    if (lane == 0) {
+#pragma unroll
+      for (int i = 0; i < 3; ++i) {
+        U.F[3 * slot + i] = f[i];
+        U.T[3 * slot + i] = t[i];
+      }
+    }
+  }
+  const unsigned ng = gsumu<32>(cnt.grid, FULL), nf = gsumu<32>(cnt.ff, FULL);
+  unsigned long long* ctr = T.sim(0).ctr;
+  if (lane == 0 && ng) atomicAdd(ctr + C_GRID_EVALS, (unsigned long long)ng);
+  if (lane == 0 && nf) atomicAdd(ctr + C_FF_EVALS, (unsigned long long)nf);
 }
 
 // Born direction 2 of one pose by a whole warp (the same terms and order as warp_reverse_born):
@@ -260,21 +379,20 @@ __device__ __forceinline__ void lean_reverse_born(const DevSystem& S, const Slot
   r[2] += (double)rs2;
 }
 
-template <typename FT, bool TORQUE>
-__global__ void __launch_bounds__(256, 4) split_rev_kernel(DevSystem S, SlotBuf B, SplitBuf U,
-                                                           unsigned long long* ctr) {
+template <typename FT, bool TORQUE, class TAB>
+__global__ void __launch_bounds__(256, sizeof(FT) == 4 ? 4 : 3) split_rev_kernel(const __grid_constant__ TAB T,
+                                                                                SlotBuf B, SplitBuf U, int set) {
   using V4 = typename Vec4<FT>::type;
   __shared__ V4 bufs[8][kSplitBuf];
   const unsigned FULL = 0xffffffffu;
   const int lane = threadIdx.x & 31;
-  const int n = U.cnt[0];
+  const int n = U.cnt[4 * set + 1], n_warps = (gridDim.x * blockDim.x) >> 5;
   unsigned nr = 0;
-  for (;;) {
-    int j = 0;
-    if (lane == 0) j = atomicAdd(U.cnt + 1, 1);
-    j = __shfl_sync(FULL, j, 0);
-    if (j >= n) break;
-    const int slot = U.list[j];
+  for (int j = (threadIdx.x >> 5) * gridDim.x + blockIdx.x; j < n;
+       j = next_item(U.cnt + 4 * set + 3, n_warps, lane)) {
+    const int slot = U.rlist[j];
+    int id = B.traj[slot];
+    const DevSystem& S = T.sys(T.locate(id));
     double r[3] = {0, 0, 0}, u[3] = {0, 0, 0};
     lean_reverse_born<FT, TORQUE>(S, B, slot, lane, bufs[threadIdx.x >> 5], r, u, nr);
     r[0] = gsum<32>(r[0], FULL);
@@ -289,95 +407,7 @@ __global__ void __launch_bounds__(256, 4) split_rev_kernel(DevSystem S, SlotBuf 
     else if (lane < 6) U.rv[6 * slot + lane] = u[lane - 3];
   }
   nr = gsumu<32>(nr, FULL);
-  if (lane == 0 && nr) atomicAdd(ctr + C_REV_EVALS, (unsigned long long)nr);
-}
-
-template <typename FT, bool TORQUE>
-__global__ void __launch_bounds__(256, 2) split_end_kernel(DevSystem S, DevSim P, SlotBuf B,
-                                                           const int* __restrict__ n_live, SplitBuf U) {
-  const BlockShared sh = block_shared_begin(S, P);
-  const int lane = threadIdx.x & 31;
-  const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, n_warps = (gridDim.x * blockDim.x) >> 5;
-  const int live = *n_live;
-  Tally tl{};
-  for (int base = warp * 32; base < live; base += n_warps * 32) {
-    const int slot = base + lane;
-    const bool own = slot < live;
-    Traj tr{};
-    tr.status = ST_EMPTY;
-    if (own) load_slot(B, slot, tr);
-    const int mode = own ? (int)U.mode[slot] : 0;
-    const bool need = mode != 0;
-    double R[9] = {1, 0, 0, 0, 1, 0, 0, 0, 1}, r = 0;
-    double F[3] = {0, 0, 0}, T[3] = {0, 0, 0};
-    if (need) {
-      quat_to_rot(tr.q, R);
-      r = norm3(tr.c[0], tr.c[1], tr.c[2]);
-#pragma unroll
-      for (int k = 0; k < 3; ++k) {
-        F[k] = U.F[3 * slot + k];
-        T[k] = U.T[3 * slot + k];
-      }
-      if (mode == 3) {
-        // the reverse-Born force on the receptor, rotated to the lab frame, acts on the ligand
-        // with the opposite sign
-        const double* rv = U.rv + 6 * slot;
-#pragma unroll
-        for (int k = 0; k < 3; ++k) F[k] = F[k] - (R[3 * k] * rv[0] + R[3 * k + 1] * rv[1] + R[3 * k + 2] * rv[2]);
-        if (TORQUE) {
-#pragma unroll
-          for (int k = 0; k < 3; ++k)
-            T[k] = T[k] - (R[3 * k] * rv[3] + R[3 * k + 1] * rv[4] + R[3 * k + 2] * rv[5]);
-        }
-      }
-    }
-    const Keyed key = traj_key(P, tr.id);
-    const uint32_t s = (uint32_t)tr.steps;
-    double cn[3] = {0, 0, 0}, qn[4] = {1, 0, 0, 0}, dt = 0;
-    bool ok = true;
-    if (need) ok = step_move<FT>(S, P, key, s, tr, R, r, F, T, cn, qn, dt);
-    int st = tr.status;
-    if (need && !ok) {
-      tl.nonfinite += 1;
-      st = ST_ERROR;
-    }
-    const bool ovl = warp_overlap(S, cn, need && ok && P.overlap, lane, sh.v);
-    if (need && ok) {
-      const double c0[3] = {tr.c[0], tr.c[1], tr.c[2]};
-      st = step_end(S, P, key, s, tr, R, cn, qn, !ovl, dt, tl);
-      if (P.stats) {
-        stats_step(S, P, tr, s, U.rprev[slot], dt, c0, R, sh.stats);
-        trace_step(P, tr, s, F, dt);
-        if (st == ST_REACTED) stats_encounter(P, tr, s, true);
-      }
-    }
-    if (need && st != ST_RUNNING) {
-      tr.status = st;
-      P.out_status[tr.id] = (int8_t)st;
-      P.out_steps[tr.id] = tr.steps;
-      P.out_returns[tr.id] = tr.rets;
-      tl.reacted += st == ST_REACTED;
-      tl.escaped += st == ST_ESCAPED;
-      tl.maxsteps += st == ST_MAXSTEPS;
-    }
-    bool dead = !own;
-    warp_refill(P, tr, dead, lane);
-    if (own) {
-      store_slot(B, slot, tr);
-      // rejected and still running: the next step starts from the same pose with these forces
-      const bool keep = need && ok && ovl && st == ST_RUNNING;
-      if (keep && mode != 2) {
-#pragma unroll
-        for (int k = 0; k < 3; ++k) {
-          U.F[3 * slot + k] = F[k];
-          U.T[3 * slot + k] = T[k];
-        }
-      }
-      U.fresh[slot] = (int8_t)keep;
-    }
-  }
-  flush_tally(P, tl, true);
-  stats_block_end(P, sh.stats);
+  if (lane == 0 && nr) atomicAdd(T.sim(0).ctr + C_REV_EVALS, (unsigned long long)nr);
 }
 
 }  // namespace bd

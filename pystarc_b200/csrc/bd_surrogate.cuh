@@ -278,6 +278,6 @@ __global__ void __launch_bounds__(256, 2) sur_end_kernel(DevSystem S, DevSim P, 
   if (lane == 0 && n_fb) atomicAdd(U.ctr + 1, (unsigned long long)n_fb);
 }
 
-__global__ void zero_int_kernel(int* p) { *p = 0; }
+static __global__ void zero_int_kernel(int* p) { *p = 0; }
 
 }  // namespace bd
