@@ -25,7 +25,9 @@
 
 namespace bd {
 
-constexpr int kSplitBuf = 128;   // candidate entries per warp (whole groups of 32 are drained)
+// Candidate entries per warp of the sweep (whole groups of 32 are drained).
+template <typename FT>
+constexpr int kSplitBuf = sizeof(FT) == 4 ? 128 : 64;
 constexpr int kStepBlock = 128;  // threads of a scalar-kernel block
 
 // Per-slot scratch of one BD step.
@@ -246,6 +248,75 @@ __global__ void __launch_bounds__(256, 2) split_fwd_kernel(const __grid_constant
   if (lane == 0 && nf) atomicAdd(ctr + C_FF_EVALS, (unsigned long long)nf);
 }
 
+// The pose of slot `slot` as the sweep of direction 2 needs it: rotation and centre in FT, and its
+// tests of receptor chunks and atoms against the ligand Born grid's margin box in the ligand frame.
+template <typename FT>
+struct RevPose {
+  using V4 = typename Vec4<FT>::type;
+  FT Rt[9], cx, cy, cz;
+
+  __device__ __forceinline__ RevPose(const SlotBuf& B, int slot) {
+    const double q[4] = {B.q[slot], B.q[B.cap + slot], B.q[2 * B.cap + slot], B.q[3 * B.cap + slot]};
+    double R[9];
+    quat_to_rot(q, R);
+#pragma unroll
+    for (int k = 0; k < 9; ++k) Rt[k] = (FT)R[k];
+    cx = (FT)B.c[slot];
+    cy = (FT)B.c[B.cap + slot];
+    cz = (FT)B.c[2 * B.cap + slot];
+  }
+
+  // Chunk k's bounding sphere reaches the box.
+  __device__ __forceinline__ bool hits(const DevSystem& S, int k) const {
+    if (k >= S.n_chunks) return false;
+    const DevGrid& g = S.lig_born;
+    const FT lox = (FT)g.lox, loy = (FT)g.loy, loz = (FT)g.loz, hix = (FT)g.hix, hiy = (FT)g.hiy, hiz = (FT)g.hiz;
+    V4 sp;
+    if constexpr (sizeof(FT) == 4) sp = S.chunks_f[k];
+    else sp = S.chunks[k];
+    const FT d0 = (FT)sp.x - cx, d1 = (FT)sp.y - cy, d2 = (FT)sp.z - cz;
+    const FT l0 = Rt[0] * d0 + Rt[3] * d1 + Rt[6] * d2;
+    const FT l1 = Rt[1] * d0 + Rt[4] * d1 + Rt[7] * d2;
+    const FT l2 = Rt[2] * d0 + Rt[5] * d1 + Rt[8] * d2;
+    const FT ex = fmax(fmax(lox - l0, l0 - hix), (FT)0);
+    const FT ey = fmax(fmax(loy - l1, l1 - hiy), (FT)0);
+    const FT ez = fmax(fmax(loz - l2, l2 - hiz), (FT)0);
+    // the radius is inflated against rounding; the extra margin covers FP32 geometry
+    const FT lim = (FT)sp.w + (sizeof(FT) == 4 ? (FT)1e-3 : (FT)1e-9);
+    return ex * ex + ey * ey + ez * ez < lim * lim;
+  }
+
+  // Receptor atom idx is charged and inside the box; e = its ligand-frame position and charge.
+  __device__ __forceinline__ bool candidate(const DevSystem& S, const SlotBuf& B, int slot, int idx, V4& e) const {
+    const DevGrid& g = S.lig_born;
+    const FT lox = (FT)g.lox, loy = (FT)g.loy, loz = (FT)g.loz, hix = (FT)g.hix, hiy = (FT)g.hiy, hiz = (FT)g.hiz;
+    V4 at;
+    if constexpr (sizeof(FT) == 4) at = S.rec_f[idx];
+    else at = S.rec[idx];
+    if (!(fabs(at.w) >= (FT)1e-9)) return false;
+    const FT d0 = (FT)at.x - cx, d1 = (FT)at.y - cy, d2 = (FT)at.z - cz;
+    const FT l0 = Rt[0] * d0 + Rt[3] * d1 + Rt[6] * d2;
+    const FT l1 = Rt[1] * d0 + Rt[4] * d1 + Rt[7] * d2;
+    const FT l2 = Rt[2] * d0 + Rt[5] * d1 + Rt[8] * d2;
+    bool cand = l0 > lox && l0 < hix && l1 > loy && l1 < hiy && l2 > loz && l2 < hiz;
+    if constexpr (sizeof(FT) == 4) {
+      // within 1e-3 A of a face the FP64 box test decides (the set of atoms is the FP64 one)
+      const float m = fminf(fminf(fminf(l0 - lox, hix - l0), fminf(l1 - loy, hiy - l1)), fminf(l2 - loz, hiz - l2));
+      if (fabsf(m) < 1e-3f) {
+        const double q[4] = {B.q[slot], B.q[B.cap + slot], B.q[2 * B.cap + slot], B.q[3 * B.cap + slot]};
+        double R[9];
+        quat_to_rot(q, R);
+        const double4 a64 = S.rec[idx];
+        const double e0 = a64.x - B.c[slot], e1 = a64.y - B.c[B.cap + slot], e2 = a64.z - B.c[2 * B.cap + slot];
+        cand = in_box(g, R[0] * e0 + R[3] * e1 + R[6] * e2, R[1] * e0 + R[4] * e1 + R[7] * e2,
+                      R[2] * e0 + R[5] * e1 + R[8] * e2);
+      }
+    }
+    e = Vec4<FT>::make(l0, l1, l2, (FT)at.w);
+    return cand;
+  }
+};
+
 // Born direction 2 of one pose by a whole warp (the same terms and order as warp_reverse_born):
 // receptor chunks culled against the ligand Born grid's margin box in the ligand frame, in-box
 // atoms gathered into `buf` and drained 32 at a time.  Adds this lane's share of the sums to
@@ -257,88 +328,29 @@ __device__ __forceinline__ void lean_reverse_born(const DevSystem& S, const Slot
   using V4 = typename Vec4<FT>::type;
   const unsigned FULL = 0xffffffffu;
   const DevGrid& g = S.lig_born;
-  FT Rt[9], cx, cy, cz;
-  {
-    const double q[4] = {B.q[slot], B.q[B.cap + slot], B.q[2 * B.cap + slot], B.q[3 * B.cap + slot]};
-    double R[9];
-    quat_to_rot(q, R);
-#pragma unroll
-    for (int k = 0; k < 9; ++k) Rt[k] = (FT)R[k];
-    cx = (FT)B.c[slot];
-    cy = (FT)B.c[B.cap + slot];
-    cz = (FT)B.c[2 * B.cap + slot];
-  }
-  const FT lox = (FT)g.lox, loy = (FT)g.loy, loz = (FT)g.loz, hix = (FT)g.hix, hiy = (FT)g.hiy, hiz = (FT)g.hiz;
-  using AT = typename Vec4<FT>::type;
-  const AT* atoms;
-  const AT* spheres;
-  if constexpr (sizeof(FT) == 4) {
-    atoms = S.rec_f;
-    spheres = S.chunks_f;
-  } else {
-    atoms = S.rec;
-    spheres = S.chunks;
-  }
+  const RevPose<FT> pose(B, slot);
   FT rs0 = 0, rs1 = 0, rs2 = 0;
   int k0 = 0, head = 0;
   unsigned hits = 0;
   bool done = false;
   for (;;) {
     // gather until the buffer has no room for another chunk, or every chunk is done
-    while (head <= kSplitBuf - 32) {
+    while (head <= kSplitBuf<FT> - 32) {
       if (!hits) {
         if (k0 >= S.n_chunks) {
           done = true;
           break;
         }
-        const int k = k0 + lane;
-        bool hit = false;
-        if (k < S.n_chunks) {
-          const AT sp = spheres[k];
-          const FT d0 = (FT)sp.x - cx, d1 = (FT)sp.y - cy, d2 = (FT)sp.z - cz;
-          const FT l0 = Rt[0] * d0 + Rt[3] * d1 + Rt[6] * d2;
-          const FT l1 = Rt[1] * d0 + Rt[4] * d1 + Rt[7] * d2;
-          const FT l2 = Rt[2] * d0 + Rt[5] * d1 + Rt[8] * d2;
-          const FT ex = fmax(fmax(lox - l0, l0 - hix), (FT)0);
-          const FT ey = fmax(fmax(loy - l1, l1 - hiy), (FT)0);
-          const FT ez = fmax(fmax(loz - l2, l2 - hiz), (FT)0);
-          // the radius is inflated against rounding; the extra margin covers FP32 geometry
-          const FT lim = (FT)sp.w + (sizeof(FT) == 4 ? (FT)1e-3 : (FT)1e-9);
-          hit = ex * ex + ey * ey + ez * ez < lim * lim;
-        }
-        hits = __ballot_sync(FULL, hit);
+        hits = __ballot_sync(FULL, pose.hits(S, k0 + lane));
         k0 += 32;
         continue;
       }
       const int kk = k0 - 32 + __ffs(hits) - 1;
       hits &= hits - 1;
-      const int idx = kk * BD_CHUNK + lane;
-      const AT at = atoms[idx];
-      FT l0 = 0, l1 = 0, l2 = 0;
-      bool cand = false;
-      if (fabs(at.w) >= (FT)1e-9) {
-        const FT d0 = (FT)at.x - cx, d1 = (FT)at.y - cy, d2 = (FT)at.z - cz;
-        l0 = Rt[0] * d0 + Rt[3] * d1 + Rt[6] * d2;
-        l1 = Rt[1] * d0 + Rt[4] * d1 + Rt[7] * d2;
-        l2 = Rt[2] * d0 + Rt[5] * d1 + Rt[8] * d2;
-        cand = l0 > lox && l0 < hix && l1 > loy && l1 < hiy && l2 > loz && l2 < hiz;
-        if constexpr (sizeof(FT) == 4) {
-          // within 1e-3 A of a face the FP64 box test decides (the set of atoms is the FP64 one)
-          const float m = fminf(fminf(fminf(l0 - lox, hix - l0), fminf(l1 - loy, hiy - l1)),
-                                fminf(l2 - loz, hiz - l2));
-          if (fabsf(m) < 1e-3f) {
-            const double q[4] = {B.q[slot], B.q[B.cap + slot], B.q[2 * B.cap + slot], B.q[3 * B.cap + slot]};
-            double R[9];
-            quat_to_rot(q, R);
-            const double4 a64 = S.rec[idx];
-            const double e0 = a64.x - B.c[slot], e1 = a64.y - B.c[B.cap + slot], e2 = a64.z - B.c[2 * B.cap + slot];
-            cand = in_box(g, R[0] * e0 + R[3] * e1 + R[6] * e2, R[1] * e0 + R[4] * e1 + R[7] * e2,
-                          R[2] * e0 + R[5] * e1 + R[8] * e2);
-          }
-        }
-      }
+      V4 ent{};
+      const bool cand = pose.candidate(S, B, slot, kk * BD_CHUNK + lane, ent);
       const unsigned m = __ballot_sync(FULL, cand);
-      if (cand) buf[head + __popc(m & ((1u << lane) - 1u))] = Vec4<FT>::make(l0, l1, l2, (FT)at.w);
+      if (cand) buf[head + __popc(m & ((1u << lane) - 1u))] = ent;
       head += __popc(m);
     }
     __syncwarp();
@@ -379,32 +391,186 @@ __device__ __forceinline__ void lean_reverse_born(const DevSystem& S, const Slot
   r[2] += (double)rs2;
 }
 
+// A product rounded by itself: never fused into the sum it goes to.
+__device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
+
+// Barrier of the `threads` threads of a block that share named barrier `id`.
+__device__ __forceinline__ void group_sync(int id, int threads) {
+  asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
+
+// Born direction 2 of one pose by W = 2, 4 or 8 warps of a block: warp gw of the group gathers
+// every W-th hit chunk, the entries land in `buf` (W * kSplitBuf of them) in the order of
+// lean_reverse_born, every thread evaluates stencils, and the sums are then taken entry by entry
+// as there, by lane e mod 32 in order: the same bits.  The force sums (r) end in warp 0 and the
+// torque sums (u) in warp 1, per lane; the caller reduces them.  `val` holds the evaluated
+// coefficient and gradient (it is `buf` itself when the positions are not needed again);
+// cnt: two rows of W counts.  Every warp of the group takes the same path (the culls and counts
+// it depends on are the same on each), so the group's barriers match.
+template <typename FT, bool TORQUE>
+__device__ __forceinline__ void group_reverse_born(const DevSystem& S, const SlotBuf& B, int slot, int lane, int gw,
+                                                   int W, int bar, typename Vec4<FT>::type* buf,
+                                                   typename Vec4<FT>::type* val, int* cnt, double r[3], double u[3],
+                                                   unsigned& nr) {
+  using V4 = typename Vec4<FT>::type;
+  const unsigned FULL = 0xffffffffu;
+  const DevGrid& g = S.lig_born;
+  const RevPose<FT> pose(B, slot);
+  const FT alpha = (FT)S.alpha;
+  FT rs0 = 0, rs1 = 0, rs2 = 0;
+  int head = 0, flip = 0;
+  // evaluate and sum the first n entries (a multiple of 32, or all of them)
+  auto drain = [&](int n) {
+    group_sync(bar, 32 * W);
+#pragma unroll 1
+    for (int e = 32 * gw + lane; e < n; e += 32 * W) {
+      const V4 v = buf[e];
+      const StencilOut<FT, 1> st = stencil<FT, 1, FT>(g, v.x, v.y, v.z);
+      val[e] = Vec4<FT>::make(-alpha * v.w * v.w, st.gx[0], st.gy[0], st.gz[0]);
+      nr += 1;
+    }
+    group_sync(bar, 32 * W);
+    if (gw == 0) {
+#pragma unroll 4
+      for (int e = lane; e < n; e += 32) {
+        const V4 v = val[e];
+        // lean_reverse_born rounds the products where it uses them twice (torque), and fuses them
+        // into the sums otherwise
+        if (TORQUE) {
+          rs0 += mul_rn(v.x, v.y);
+          rs1 += mul_rn(v.x, v.z);
+          rs2 += mul_rn(v.x, v.w);
+        } else {
+          rs0 = fma(v.x, v.y, rs0);
+          rs1 = fma(v.x, v.z, rs1);
+          rs2 = fma(v.x, v.w, rs2);
+        }
+      }
+    }
+    if (TORQUE && gw == 1) {
+#pragma unroll 4
+      for (int e = lane; e < n; e += 32) {
+        const V4 v = val[e], p = buf[e];
+        const FT g0 = mul_rn(v.x, v.y), g1 = mul_rn(v.x, v.z), g2 = mul_rn(v.x, v.w);
+        const double x = (double)p.x, y = (double)p.y, z = (double)p.z;
+        u[0] += y * (double)g2 - z * (double)g1;
+        u[1] += z * (double)g0 - x * (double)g2;
+        u[2] += x * (double)g1 - y * (double)g0;
+      }
+    }
+    group_sync(bar, 32 * W);
+  };
+  for (int c0 = 0; c0 < S.n_chunks; c0 += 1024) {
+    // lane l keeps the hit mask of chunks c0 + 32 l .. + 31
+    unsigned mine = 0;
+    const int n_mask = min(32, (S.n_chunks - c0 + 31) / 32);
+    for (int l = 0; l < n_mask; ++l) {
+      const unsigned m = __ballot_sync(FULL, pose.hits(S, c0 + 32 * l + lane));
+      if (lane == l) mine = m;
+    }
+    int before = __popc(mine);  // exclusive prefix of the hit counts
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int t = __shfl_up_sync(FULL, before, o);
+      if (lane >= o) before += t;
+    }
+    const int H = __shfl_sync(FULL, before, 31);
+    before -= __popc(mine);
+    for (int h0 = 0; h0 < H; h0 += W) {
+      const int h = h0 + gw;
+      V4 ent{};
+      bool cand = false;
+      if (h < H) {
+        // the chunk of hit h: its mask's lane, then the bit with that many hits below it
+        const unsigned has = __ballot_sync(FULL, before <= h && h < before + __popc(mine));
+        const int src = __ffs(has) - 1;
+        const unsigned m = __shfl_sync(FULL, mine, src);
+        const int nth = h - __shfl_sync(FULL, before, src);
+        const unsigned at =
+            __ballot_sync(FULL, ((m >> lane) & 1u) && __popc(m & ((1u << lane) - 1u)) == nth);
+        cand = pose.candidate(S, B, slot, (c0 + 32 * src + __ffs(at) - 1) * BD_CHUNK + lane, ent);
+      }
+      const unsigned m = __ballot_sync(FULL, cand);
+      if (lane == 0) cnt[flip * 8 + gw] = __popc(m);
+      group_sync(bar, 32 * W);
+      int at = head, total = 0;
+      for (int w = 0; w < W; ++w) {
+        const int k = cnt[flip * 8 + w];
+        if (w < gw) at += k;
+        total += k;
+      }
+      flip ^= 1;
+      if (cand) buf[at + __popc(m & ((1u << lane) - 1u))] = ent;
+      head += total;
+      if (head > (kSplitBuf<FT> - 32) * W) {  // no room for another round
+        const int n = head & ~31, rem = head - n;
+        drain(n);
+        V4 keep{};
+        if (gw == 0 && lane < rem) keep = buf[n + lane];
+        group_sync(bar, 32 * W);
+        if (gw == 0 && lane < rem) buf[lane] = keep;
+        head = rem;
+      }
+    }
+  }
+  drain(head);
+  r[0] = (double)rs0;
+  r[1] = (double)rs1;
+  r[2] = (double)rs2;
+}
+
+// Warps per pose of the sweep for a list of n poses on n_warps resident warps: a list that leaves
+// warps idle gives each pose more of them.  One warp takes 20-40 us for a pose in contact (a serial
+// chain of chunk gathers and stencil drains), so a short list is bound by that latency: 1,000
+// trajectories FP64 took 89 us a sweep with one warp per pose, and the whole run's GPU time fell
+// from 120 to 40 ms with eight; 8,000 mixed 200 -> 136 ms, 30,011 FP64 170 -> 147 ms.  Lines twice
+// and four times as far out are no better (8,000: 142 and 134 ms; 30,011 FP64: 172 and 168 ms).
+__device__ __forceinline__ int rev_warps(int n, int n_warps) {
+  return n * 4 <= n_warps ? 8 : n * 2 <= n_warps ? 4 : n <= n_warps ? 2 : 1;
+}
+
+// FP32: capped at 64 registers, 32 warps per SM.  FP64: at 128; the cap of 80 spills 388 bytes and
+// measured slower (30,011 FP64 trajectories: 147 against 136 ms of GPU time).
 template <typename FT, bool TORQUE, class TAB>
-__global__ void __launch_bounds__(256, sizeof(FT) == 4 ? 4 : 3) split_rev_kernel(const __grid_constant__ TAB T,
+__global__ void __launch_bounds__(256, sizeof(FT) == 4 ? 4 : 2) split_rev_kernel(const __grid_constant__ TAB T,
                                                                                 SlotBuf B, SplitBuf U, int set) {
   using V4 = typename Vec4<FT>::type;
-  __shared__ V4 bufs[8][kSplitBuf];
+  __shared__ V4 bufs[8][kSplitBuf<FT>];
+  __shared__ V4 vals[TORQUE ? 8 : 1][TORQUE ? kSplitBuf<FT> : 1];
+  __shared__ int cnts[4][16];
   const unsigned FULL = 0xffffffffu;
-  const int lane = threadIdx.x & 31;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int n = U.cnt[4 * set + 1], n_warps = (gridDim.x * blockDim.x) >> 5;
+  const int W = rev_warps(n, n_warps);
+  const int gw = warp & (W - 1), grp = warp / W;  // warp of the group, group of the block
   unsigned nr = 0;
-  for (int j = (threadIdx.x >> 5) * gridDim.x + blockIdx.x; j < n;
-       j = next_item(U.cnt + 4 * set + 3, n_warps, lane)) {
+  for (int j = grp * gridDim.x + blockIdx.x; j < n;
+       j = W > 1 ? j + n_warps / W : next_item(U.cnt + 4 * set + 3, n_warps, lane)) {
     const int slot = U.rlist[j];
     int id = B.traj[slot];
     const DevSystem& S = T.sys(T.locate(id));
     double r[3] = {0, 0, 0}, u[3] = {0, 0, 0};
-    lean_reverse_born<FT, TORQUE>(S, B, slot, lane, bufs[threadIdx.x >> 5], r, u, nr);
-    r[0] = gsum<32>(r[0], FULL);
-    r[1] = gsum<32>(r[1], FULL);
-    r[2] = gsum<32>(r[2], FULL);
-    if (TORQUE) {
+    if (W == 1) {
+      lean_reverse_born<FT, TORQUE>(S, B, slot, lane, bufs[warp], r, u, nr);
+    } else {
+      V4* buf = bufs[grp * W];
+      group_reverse_born<FT, TORQUE>(S, B, slot, lane, gw, W, 1 + grp, buf, TORQUE ? vals[grp * W] : buf, cnts[grp], r,
+                                     u, nr);
+    }
+    if (gw == 0) {
+      r[0] = gsum<32>(r[0], FULL);
+      r[1] = gsum<32>(r[1], FULL);
+      r[2] = gsum<32>(r[2], FULL);
+      if (lane < 3) U.rv[6 * slot + lane] = r[lane];
+      if (!TORQUE && lane < 3) U.rv[6 * slot + 3 + lane] = 0.0;
+    }
+    if (TORQUE && gw == (W > 1 ? 1 : 0)) {
       u[0] = gsum<32>(u[0], FULL);
       u[1] = gsum<32>(u[1], FULL);
       u[2] = gsum<32>(u[2], FULL);
+      if (lane < 3) U.rv[6 * slot + 3 + lane] = u[lane];
     }
-    if (lane < 3) U.rv[6 * slot + lane] = r[lane];
-    else if (lane < 6) U.rv[6 * slot + lane] = u[lane - 3];
   }
   nr = gsumu<32>(nr, FULL);
   if (lane == 0 && nr) atomicAdd(T.sim(0).ctr + C_REV_EVALS, (unsigned long long)nr);

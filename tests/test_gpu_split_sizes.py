@@ -1,7 +1,7 @@
 """The split stepper at the sizes where its lists and pools can go wrong, against the fused stepper.
 
-One slot, one more than a warp, one more than a block of the scalar kernel, and more slots than
-the force kernels have warps; launches of one step (begin and end without a middle kernel), of an
+One slot, one more than a warp, one more than a block of the scalar kernel, sizes at which eight,
+four and two warps share a pose of the sweep, and more slots than the force kernels have warps; launches of one step (begin and end without a middle kernel), of an
 odd and of an even number of steps; pools with and without refill.  In FP64 and in mixed precision
 both steppers sum every pose's terms in the same order, so outcomes are equal, not close.
 """
@@ -15,7 +15,8 @@ from tests.test_gpu_stepper import make_sim
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("n,slots,K", [(1, 1, 1), (33, 33, 3), (129, 129, 1), (400, 33, 2), (6001, 6001, 16)])
+@pytest.mark.parametrize("n,slots,K", [(1, 1, 1), (33, 33, 3), (129, 129, 1), (400, 33, 2), (1500, 1500, 5), (3001, 3001, 4),
+                                       (6001, 6001, 16)])
 @pytest.mark.parametrize("precision", ["fp64", "mixed"])
 @pytest.mark.parametrize("sysname", ["c2", "c3"])
 def test_split_outcomes_equal_the_fused_steppers(n, slots, K, precision, sysname):
