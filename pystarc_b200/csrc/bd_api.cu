@@ -54,7 +54,8 @@ struct BdHandle {
   bool fp_set = false;
   int n_pairs = 0, n_needed = 1;
   double rx_rec[BD_MAX_PAIRS][3], rx_body[BD_MAX_PAIRS][3], rx_cut[BD_MAX_PAIRS], rx_deff[BD_MAX_PAIRS];
-  bool dirty = true;
+  bool dirty = true;     // the device system is to be rebuilt
+  bool rx_dirty = false; // only the reaction tables changed since it was built
   // device system
   DevSystem S{};
   std::vector<void*> sys_allocs;
@@ -67,7 +68,12 @@ struct BdHandle {
   int* d_live = nullptr;  // [2]
   int cur = 0;
   unsigned long long* d_ctr = nullptr;
-  std::vector<void*> sim_allocs;
+  struct SimBlock {
+    void* p;
+    size_t bytes;
+    bool used;
+  };
+  std::vector<SimBlock> sim_blocks;  // device buffers of the configured run (sim_alloc)
   int group = 8, block = 128;
   bool launch_user = false;
   int layout = BD_LAYOUT_DEFAULT;
@@ -83,9 +89,9 @@ struct BdHandle {
   cudaStream_t side = nullptr;  // capture only: the force kernel that runs beside the other
   cudaEvent_t fork = nullptr, join = nullptr;
   unsigned long long* sur_ctr_host_base = nullptr;
-  // graphs: [cur][steps] cache
+  // graphs, one per slot buffer, and the bytes of everything that was captured into them
   cudaGraphExec_t graph[2] = {nullptr, nullptr};
-  int graph_K = -1, graph_G = -1, graph_B = -1, graph_prec = -1, graph_torque = -1;
+  std::vector<unsigned char> graph_key;
 };
 
 namespace {
@@ -113,6 +119,30 @@ int dev_alloc(BdHandle* h, std::vector<void*>& list, void** p, size_t bytes) {
   CK(h, cudaMalloc(p, bytes ? bytes : 16));
   list.push_back(*p);
   return BD_OK;
+}
+
+// A device buffer of the configured run.  A run with the sizes of the one before it takes that
+// one's buffers: freeing and allocating the pool again took 6 ms a run for two spheres (100,000
+// trajectories).  bd_sim_configure gives back what the new run did not take.
+int sim_alloc(BdHandle* h, void** p, size_t bytes) {
+  if (!bytes) bytes = 16;
+  for (auto& b : h->sim_blocks)
+    if (!b.used && b.bytes == bytes) {
+      b.used = true;
+      *p = b.p;
+      return BD_OK;
+    }
+  CK(h, cudaMalloc(p, bytes));
+  h->sim_blocks.push_back({*p, bytes, true});
+  return BD_OK;
+}
+
+// Free the buffers that no sim_alloc has taken since they were marked unused.
+void free_unused(BdHandle* h) {
+  auto& v = h->sim_blocks;
+  for (auto& b : v)
+    if (!b.used) cudaFree(b.p);
+  v.erase(std::remove_if(v.begin(), v.end(), [](const BdHandle::SimBlock& b) { return !b.used; }), v.end());
 }
 
 void free_list(std::vector<void*>& list) {
@@ -374,9 +404,47 @@ bool same_lattice(const GridHost& a, const GridHost& b) {
   return true;
 }
 
-// Build the device-side system: grid selection rules, uploads, receptor chunks.
+// The reaction tables of the device system (they travel with the kernels' parameters).
+int set_reaction_tables(BdHandle* h, DevSystem& S) {
+  S.n_pairs = h->n_pairs;
+  S.n_needed = h->n_needed;
+  for (int p = 0; p < h->n_pairs; ++p) {
+    for (int k = 0; k < 3; ++k) {
+      S.rx_rec[p][k] = h->rx_rec[p][k];
+      S.rx_body[p][k] = h->rx_body[p][k];
+    }
+    S.rx_cut[p] = h->rx_cut[p];
+    S.rx_deff[p] = h->rx_deff[p];
+  }
+  S.sm = 0;
+  S.n_states = 0;
+  S.terminal = 0;
+  if (h->sm_n > 0) {
+    if (h->sm_n != h->n_pairs)
+      return fail(h, BD_ERR_ARG, "state-machine reactions: %d reactions but %d reaction pairs (one pair each)",
+                  h->sm_n, h->n_pairs);
+    S.sm = 1;
+    S.n_states = h->sm_states;
+    S.terminal = h->sm_terminal;
+    for (int p = 0; p < h->sm_n; ++p) {
+      S.rx_before[p] = h->sm_before[p];
+      S.rx_after[p] = h->sm_after[p];
+    }
+  }
+  return BD_OK;
+}
+
+// Build the device-side system: grid selection rules, uploads, receptor chunks.  Every run sets the
+// reactions anew; where nothing else changed the grids and tables on the device stay (rebuilding
+// them took 60-90 ms of each run on 193^3 grids).
 int finalize(BdHandle* h) {
-  if (!h->dirty) return BD_OK;
+  if (!h->dirty) {
+    if (h->rx_dirty) {
+      if (int rc = set_reaction_tables(h, h->S)) return rc;
+      h->rx_dirty = false;
+    }
+    return BD_OK;
+  }
   CK(h, cudaSetDevice(h->device));
   CK(h, cudaDeviceSynchronize());
   free_tex(h->sys_tex);
@@ -401,8 +469,11 @@ int finalize(BdHandle* h) {
     S.inv_fpe = 1.0 / fp.four_pi_eps;
   }
   // grids: finest first (stable on the x spacing), reference dropping rules
-  std::vector<GridHost> el = h->grids[BD_GRID_ELEC], bo = h->grids[BD_GRID_BORN], lb = h->grids[BD_GRID_LIG_BORN];
-  auto finer = [](const GridHost& a, const GridHost& b) { return a.sp[0] < b.sp[0]; };
+  std::vector<const GridHost*> el, bo, lb;
+  for (const GridHost& g : h->grids[BD_GRID_ELEC]) el.push_back(&g);
+  for (const GridHost& g : h->grids[BD_GRID_BORN]) bo.push_back(&g);
+  for (const GridHost& g : h->grids[BD_GRID_LIG_BORN]) lb.push_back(&g);
+  auto finer = [](const GridHost* a, const GridHost* b) { return a->sp[0] < b->sp[0]; };
   std::stable_sort(el.begin(), el.end(), finer);
   std::stable_sort(bo.begin(), bo.end(), finer);
   std::stable_sort(lb.begin(), lb.end(), finer);
@@ -413,29 +484,27 @@ int finalize(BdHandle* h) {
   S.n_elec = (int)el.size();
   for (int k = 0; k < S.n_elec; ++k) {
     const float* p;
-    int rc = upload_floats(h, el[k].data.data(), el[k].data.size(), &p);
+    int rc = upload_floats(h, el[k]->data.data(), el[k]->data.size(), &p);
     if (rc) return rc;
-    grid_to_dev(el[k], p, 1, S.elec[k]);
+    grid_to_dev(*el[k], p, 1, S.elec[k]);
   }
   S.has_born = !bo.empty();
   if (S.has_born) {
     const float* p;
-    int rc = upload_floats(h, bo[0].data.data(), bo[0].data.size(), &p);
+    int rc = upload_floats(h, bo[0]->data.data(), bo[0]->data.size(), &p);
     if (rc) return rc;
-    grid_to_dev(bo[0], p, 1, S.born);
-    if (S.n_elec > 0 && same_lattice(el[0], bo[0])) {
-      std::vector<float> il(2 * el[0].data.size());
-      for (size_t i = 0; i < el[0].data.size(); ++i) {
-        il[2 * i] = el[0].data[i];
-        il[2 * i + 1] = bo[0].data[i];
-      }
-      rc = upload_floats(h, il.data(), il.size(), &p);
-      if (rc) return rc;
-      grid_to_dev(el[0], p, 2, S.pair);
+    grid_to_dev(*bo[0], p, 1, S.born);
+    if (S.n_elec > 0 && same_lattice(*el[0], *bo[0])) {
+      const size_t nodes = el[0]->data.size();
+      void* il = nullptr;
+      if ((rc = dev_alloc(h, h->sys_allocs, &il, 2 * nodes * sizeof(float)))) return rc;
+      pair_kernel<<<h->n_sm * 8, 256>>>(S.elec[0].data, S.born.data, (float2*)il, (long)nodes);
+      CK(h, cudaGetLastError());
+      grid_to_dev(*el[0], (const float*)il, 2, S.pair);
       S.paired = 1;
       // linear textures address at most 2^27 elements
-      if ((h->layout & BD_LAYOUT_PTEX_2) && el[0].data.size() <= (size_t)(1 << 27))
-        if ((rc = float2_texture(h, (void*)p, el[0].data.size(), &S.pair.ptex))) return rc;
+      if ((h->layout & BD_LAYOUT_PTEX_2) && nodes <= (size_t)(1 << 27))
+        if ((rc = float2_texture(h, il, nodes, &S.pair.ptex))) return rc;
     }
   }
   if (h->layout & BD_LAYOUT_WINDOWS_1) {
@@ -547,9 +616,9 @@ int finalize(BdHandle* h) {
   // Born direction 2 needs the ligand Born grid, receptor atoms and alpha > 1e-12 (gpu_batch_engine.py:583-590)
   if (!lb.empty() && nr > 0 && fp.alpha > 1e-12) {
     const float* p;
-    int rc = upload_floats(h, lb[0].data.data(), lb[0].data.size(), &p);
+    int rc = upload_floats(h, lb[0]->data.data(), lb[0]->data.size(), &p);
     if (rc) return rc;
-    grid_to_dev(lb[0], p, 1, S.lig_born);
+    grid_to_dev(*lb[0], p, 1, S.lig_born);
     if (h->layout & BD_LAYOUT_WINDOWS_1)
       if ((rc = add_window(h, S.lig_born))) return rc;
     if ((h->layout & BD_LAYOUT_CUBES_1) &&
@@ -568,34 +637,13 @@ int finalize(BdHandle* h) {
                  mz = std::max(std::fabs(g.loz), std::fabs(g.hiz));
     S.lig_born_rho = std::sqrt(mx * mx + my * my + mz * mz) * (1 + 1e-12) + 1e-9;
   }
-  // reactions
-  S.n_pairs = h->n_pairs;
-  S.n_needed = h->n_needed;
-  for (int p = 0; p < h->n_pairs; ++p) {
-    for (int k = 0; k < 3; ++k) {
-      S.rx_rec[p][k] = h->rx_rec[p][k];
-      S.rx_body[p][k] = h->rx_body[p][k];
-    }
-    S.rx_cut[p] = h->rx_cut[p];
-    S.rx_deff[p] = h->rx_deff[p];
-  }
-  if (h->sm_n > 0) {
-    if (h->sm_n != h->n_pairs)
-      return fail(h, BD_ERR_ARG, "state-machine reactions: %d reactions but %d reaction pairs (one pair each)",
-                  h->sm_n, h->n_pairs);
-    S.sm = 1;
-    S.n_states = h->sm_states;
-    S.terminal = h->sm_terminal;
-    for (int p = 0; p < h->sm_n; ++p) {
-      S.rx_before[p] = h->sm_before[p];
-      S.rx_after[p] = h->sm_after[p];
-    }
-  }
+  if (int rc = set_reaction_tables(h, S)) return rc;
   CK(h, cudaDeviceSynchronize());  // window copies are built on the legacy stream
   S.terms = h->terms;
   h->S = S;
   h->dirty = false;
-  h->graph_K = -1;  // system changed: rebuild graphs
+  h->rx_dirty = false;
+  h->graph_key.clear();  // system changed: rebuild graphs
   return BD_OK;
 }
 
@@ -739,7 +787,10 @@ int resident_blocks(BdHandle* h, int G, void* fn, size_t smem) {
 size_t stepper_smem(const DevSystem& S, const DevSim& P, void* fn) {
   size_t b = S.rec_in_smem ? (size_t)(S.n_rec_pad + S.n_chunks) * sizeof(float4) : 0;
   if (P.stats) b += (size_t)SH_NUM * sizeof(unsigned);
-  if (fn) cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)b);
+  // raised, never lowered: a graph captured earlier may hold a launch that needs more
+  cudaFuncAttributes a;
+  if (fn && cudaFuncGetAttributes(&a, fn) == cudaSuccess && (int)b > a.maxDynamicSharedSizeBytes)
+    cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)b);
   return b;
 }
 
@@ -780,7 +831,7 @@ int bd_destroy(BdHandle* h) {
     if (g) cudaGraphExecDestroy(g);
   free_tex(h->sys_tex);
   free_list(h->sys_allocs);
-  free_list(h->sim_allocs);
+  for (auto& b : h->sim_blocks) cudaFree(b.p);
   if (h->fork) cudaEventDestroy(h->fork);
   if (h->join) cudaEventDestroy(h->join);
   if (h->side) cudaStreamDestroy(h->side);
@@ -877,7 +928,7 @@ int bd_set_reactions(BdHandle* h, int n_pairs, const double* rec_xyz, const doub
     h->rx_cut[p] = cut[p];
     h->rx_deff[p] = d_eff[p];
   }
-  h->dirty = true;
+  h->rx_dirty = true;
   return BD_OK;
 }
 
@@ -942,7 +993,6 @@ int bd_set_launch(BdHandle* h, int group, int block) {
   if (group) h->group = group;
   if (block) h->block = block;
   h->launch_user = group != 0 || h->launch_user;
-  h->graph_K = -1;
   return BD_OK;
 }
 
@@ -960,7 +1010,7 @@ int bd_set_layout(BdHandle* h, int flags) {
 
 int bd_sim_set_surrogate(BdHandle* h, BdMlp* m, const BdSurrogateParams* p) {
   if (!h) return BD_ERR_ARG;
-  h->graph_K = -1;  // the step sequence changes
+  if (m || h->sur) h->graph_key.clear();  // the step sequence changes
   if (!m) {
     h->sur = nullptr;
     return BD_OK;
@@ -1023,7 +1073,7 @@ int bd_set_reaction_states(BdHandle* h, int n_pairs, const int32_t* state_before
   h->sm_n = n_pairs;
   h->sm_states = n_pairs > 0 ? n_states : 0;
   h->sm_terminal = term;
-  h->dirty = true;
+  h->rx_dirty = true;
   return BD_OK;
 }
 
@@ -1075,6 +1125,10 @@ int bd_get_launch(BdHandle* h, int* group, int* block, int* grid) {
   return BD_OK;
 }
 
+namespace {
+int ensure_split_buffers(BdHandle* h);
+}
+
 int bd_sim_configure(BdHandle* h, const BdSimParams* p) {
   bd::NvtxRange nvtx("bd_sim_configure");
   if (!h || !p) return fail(h, BD_ERR_ARG, "bd_sim_configure: NULL");
@@ -1095,7 +1149,7 @@ int bd_sim_configure(BdHandle* h, const BdSimParams* p) {
   if (rc) return rc;
   CK(h, cudaSetDevice(h->device));
   CK(h, cudaDeviceSynchronize());
-  free_list(h->sim_allocs);
+  for (auto& b : h->sim_blocks) b.used = false;
   h->sim_ready = false;
   h->sur_cap = 0;
   h->sur_buf = SurBuf{};
@@ -1115,42 +1169,42 @@ int bd_sim_configure(BdHandle* h, const BdSimParams* p) {
   for (int b = 0; b < 2; ++b) {
     SlotBuf& B = h->buf[b];
     void* q;
-    if ((rc = dev_alloc(h, h->sim_allocs, &q, 3 * (size_t)C * sizeof(double)))) return rc;
+    if ((rc = sim_alloc(h, &q, 3 * (size_t)C * sizeof(double)))) return rc;
     B.c = (double*)q;
-    if ((rc = dev_alloc(h, h->sim_allocs, &q, 4 * (size_t)C * sizeof(double)))) return rc;
+    if ((rc = sim_alloc(h, &q, 4 * (size_t)C * sizeof(double)))) return rc;
     B.q = (double*)q;
-    if ((rc = dev_alloc(h, h->sim_allocs, &q, (size_t)C * sizeof(int)))) return rc;
+    if ((rc = sim_alloc(h, &q, (size_t)C * sizeof(int)))) return rc;
     B.traj = (int*)q;
-    if ((rc = dev_alloc(h, h->sim_allocs, &q, (size_t)C * sizeof(int)))) return rc;
+    if ((rc = sim_alloc(h, &q, (size_t)C * sizeof(int)))) return rc;
     B.steps = (int*)q;
-    if ((rc = dev_alloc(h, h->sim_allocs, &q, (size_t)C * sizeof(int)))) return rc;
+    if ((rc = sim_alloc(h, &q, (size_t)C * sizeof(int)))) return rc;
     B.rets = (int*)q;
-    if ((rc = dev_alloc(h, h->sim_allocs, &q, (size_t)C))) return rc;
+    if ((rc = sim_alloc(h, &q, (size_t)C))) return rc;
     B.status = (int8_t*)q;
-    if ((rc = dev_alloc(h, h->sim_allocs, &q, (size_t)C))) return rc;
+    if ((rc = sim_alloc(h, &q, (size_t)C))) return rc;
     B.state = (int8_t*)q;
     B.cap = C;
   }
   void* q;
-  if ((rc = dev_alloc(h, h->sim_allocs, &q, 2 * sizeof(int)))) return rc;
+  if ((rc = sim_alloc(h, &q, 2 * sizeof(int)))) return rc;
   h->d_live = (int*)q;
-  if ((rc = dev_alloc(h, h->sim_allocs, &q, C_NUM * sizeof(unsigned long long)))) return rc;
+  if ((rc = sim_alloc(h, &q, C_NUM * sizeof(unsigned long long)))) return rc;
   h->d_ctr = (unsigned long long*)q;
   DevSim& P = h->P;
   sim_constants(p, h->S, P);
   P.ctr = h->d_ctr;
-  if ((rc = dev_alloc(h, h->sim_allocs, &q, (size_t)p->n_traj))) return rc;
+  if ((rc = sim_alloc(h, &q, (size_t)p->n_traj))) return rc;
   P.out_status = (int8_t*)q;
-  if ((rc = dev_alloc(h, h->sim_allocs, &q, (size_t)p->n_traj * sizeof(int)))) return rc;
+  if ((rc = sim_alloc(h, &q, (size_t)p->n_traj * sizeof(int)))) return rc;
   P.out_steps = (int*)q;
-  if ((rc = dev_alloc(h, h->sim_allocs, &q, (size_t)p->n_traj * sizeof(int)))) return rc;
+  if ((rc = sim_alloc(h, &q, (size_t)p->n_traj * sizeof(int)))) return rc;
   P.out_returns = (int*)q;
   if (p->stats) {
     const size_t n = (size_t)p->n_traj;
     DevStats& st = P.st;
     auto dbl = [&](double** out, size_t k) {
       void* v;
-      int r = dev_alloc(h, h->sim_allocs, &v, k * sizeof(double));
+      int r = sim_alloc(h, &v, k * sizeof(double));
       *out = (double*)v;
       return r;
     };
@@ -1158,13 +1212,13 @@ int bd_sim_configure(BdHandle* h, const BdSimParams* p) {
         (rc = dbl(&st.nm_c, 3 * n)) || (rc = dbl(&st.nm_q, 4 * n)) || (rc = dbl(&st.total_time, n)) ||
         (rc = dbl(&st.enc_c, 3 * n)) || (rc = dbl(&st.enc_q, 4 * n)))
       return rc;
-    if ((rc = dev_alloc(h, h->sim_allocs, &q, n * sizeof(int)))) return rc;
+    if ((rc = sim_alloc(h, &q, n * sizeof(int)))) return rc;
     st.step_at_min = (int*)q;
-    if ((rc = dev_alloc(h, h->sim_allocs, &q, n * sizeof(int)))) return rc;
+    if ((rc = sim_alloc(h, &q, n * sizeof(int)))) return rc;
     st.enc_step = (int*)q;
-    if ((rc = dev_alloc(h, h->sim_allocs, &q, n))) return rc;
+    if ((rc = sim_alloc(h, &q, n))) return rc;
     st.bridge = (int8_t*)q;
-    if ((rc = dev_alloc(h, h->sim_allocs, &q, SH_NUM * sizeof(unsigned long long)))) return rc;
+    if ((rc = sim_alloc(h, &q, SH_NUM * sizeof(unsigned long long)))) return rc;
     st.hist = (unsigned long long*)q;
     // bin edges as numpy.linspace builds them: start + i * (stop - start) / (num - 1), last = stop
     std::vector<double> edges(ST_RAD_BINS + 1 + ST_TRANS + 1 + ST_MILESTONES);
@@ -1178,23 +1232,25 @@ int bd_sim_configure(BdHandle* h, const BdSimParams* p) {
     const double dm = (p->r_escape - p->r_start) / (ST_MILESTONES - 1);
     for (int i = 0; i < ST_MILESTONES; ++i) mr[i] = i * dm + p->r_start;
     mr[ST_MILESTONES - 1] = p->r_escape;
-    if ((rc = dev_alloc(h, h->sim_allocs, &q, edges.size() * sizeof(double)))) return rc;
+    if ((rc = sim_alloc(h, &q, edges.size() * sizeof(double)))) return rc;
     CK(h, cudaMemcpy(q, edges.data(), edges.size() * sizeof(double), cudaMemcpyHostToDevice));
     st.rad_edges = (const double*)q;
     st.trans_edges = st.rad_edges + ST_RAD_BINS + 1;
     st.ms_radii = st.trans_edges + ST_TRANS + 1;
     P.stats = 1;
     if (p->trace_capacity > 0) {
-      if ((rc = dev_alloc(h, h->sim_allocs, &q, (size_t)p->trace_capacity * 8 * sizeof(double)))) return rc;
+      if ((rc = sim_alloc(h, &q, (size_t)p->trace_capacity * 8 * sizeof(double)))) return rc;
       P.trace_path = (double*)q;
-      if ((rc = dev_alloc(h, h->sim_allocs, &q, (size_t)p->trace_capacity * 6 * sizeof(double)))) return rc;
+      if ((rc = sim_alloc(h, &q, (size_t)p->trace_capacity * 6 * sizeof(double)))) return rc;
       P.trace_energy = (double*)q;
       P.trace_cap = p->trace_capacity;
       P.save_interval = p->save_interval;
     }
   }
+  if (!h->sur && G == BD_GROUP_SPLIT)
+    if ((rc = ensure_split_buffers(h))) return rc;
+  free_unused(h);
   h->sim_ready = true;
-  h->graph_K = -1;
   return BD_OK;
 }
 
@@ -1260,25 +1316,25 @@ int ensure_surrogate_buffers(BdHandle* h) {
   SurBuf& U = h->sur_buf;
   void* q;
   int rc;
-  if ((rc = dev_alloc(h, h->sim_allocs, &q, 3 * (size_t)C * sizeof(double)))) return rc;
+  if ((rc = sim_alloc(h, &q, 3 * (size_t)C * sizeof(double)))) return rc;
   U.F = (double*)q;
-  if ((rc = dev_alloc(h, h->sim_allocs, &q, 3 * (size_t)C * sizeof(double)))) return rc;
+  if ((rc = sim_alloc(h, &q, 3 * (size_t)C * sizeof(double)))) return rc;
   U.T = (double*)q;
-  if ((rc = dev_alloc(h, h->sim_allocs, &q, (size_t)C))) return rc;
+  if ((rc = sim_alloc(h, &q, (size_t)C))) return rc;
   U.mode = (int8_t*)q;
-  if ((rc = dev_alloc(h, h->sim_allocs, &q, (size_t)C))) return rc;
+  if ((rc = sim_alloc(h, &q, (size_t)C))) return rc;
   U.fresh = (int8_t*)q;
-  if ((rc = dev_alloc(h, h->sim_allocs, &q, (size_t)C * sizeof(int)))) return rc;
+  if ((rc = sim_alloc(h, &q, (size_t)C * sizeof(int)))) return rc;
   U.row = (int*)q;
-  if ((rc = dev_alloc(h, h->sim_allocs, &q, (size_t)C * kSurInPad * 2))) return rc;
+  if ((rc = sim_alloc(h, &q, (size_t)C * kSurInPad * 2))) return rc;
   U.X = (__nv_bfloat16*)q;
-  if ((rc = dev_alloc(h, h->sim_allocs, &q, (size_t)C * kSurOut * sizeof(float)))) return rc;
+  if ((rc = sim_alloc(h, &q, (size_t)C * kSurOut * sizeof(float)))) return rc;
   U.mean = (const float*)q;
-  if ((rc = dev_alloc(h, h->sim_allocs, &q, (size_t)C * kSurOut * sizeof(float)))) return rc;
+  if ((rc = sim_alloc(h, &q, (size_t)C * kSurOut * sizeof(float)))) return rc;
   U.spread = (const float*)q;
-  if ((rc = dev_alloc(h, h->sim_allocs, &q, sizeof(int)))) return rc;
+  if ((rc = sim_alloc(h, &q, sizeof(int)))) return rc;
   U.n_rows = (int*)q;
-  if ((rc = dev_alloc(h, h->sim_allocs, &q, 2 * sizeof(unsigned long long)))) return rc;
+  if ((rc = sim_alloc(h, &q, 2 * sizeof(unsigned long long)))) return rc;
   U.ctr = (unsigned long long*)q;
   CK(h, cudaMemset(U.X, 0, (size_t)C * kSurInPad * 2));
   CK(h, cudaMemset(U.ctr, 0, 2 * sizeof(unsigned long long)));
@@ -1328,21 +1384,21 @@ int ensure_split_buffers(BdHandle* h) {
   SplitBuf& U = h->split_buf;
   void* q;
   int rc;
-  if ((rc = dev_alloc(h, h->sim_allocs, &q, 3 * (size_t)C * sizeof(double)))) return rc;
+  if ((rc = sim_alloc(h, &q, 3 * (size_t)C * sizeof(double)))) return rc;
   U.F = (double*)q;
-  if ((rc = dev_alloc(h, h->sim_allocs, &q, 3 * (size_t)C * sizeof(double)))) return rc;
+  if ((rc = sim_alloc(h, &q, 3 * (size_t)C * sizeof(double)))) return rc;
   U.T = (double*)q;
-  if ((rc = dev_alloc(h, h->sim_allocs, &q, 6 * (size_t)C * sizeof(double)))) return rc;
+  if ((rc = sim_alloc(h, &q, 6 * (size_t)C * sizeof(double)))) return rc;
   U.rv = (double*)q;
-  if ((rc = dev_alloc(h, h->sim_allocs, &q, (size_t)C * sizeof(double)))) return rc;
+  if ((rc = sim_alloc(h, &q, (size_t)C * sizeof(double)))) return rc;
   U.rprev = (double*)q;
-  if ((rc = dev_alloc(h, h->sim_allocs, &q, (size_t)C))) return rc;
+  if ((rc = sim_alloc(h, &q, (size_t)C))) return rc;
   U.mode = (int8_t*)q;
-  if ((rc = dev_alloc(h, h->sim_allocs, &q, (size_t)C * sizeof(int)))) return rc;
+  if ((rc = sim_alloc(h, &q, (size_t)C * sizeof(int)))) return rc;
   U.flist = (int*)q;
-  if ((rc = dev_alloc(h, h->sim_allocs, &q, (size_t)C * sizeof(int)))) return rc;
+  if ((rc = sim_alloc(h, &q, (size_t)C * sizeof(int)))) return rc;
   U.rlist = (int*)q;
-  if ((rc = dev_alloc(h, h->sim_allocs, &q, 8 * sizeof(int)))) return rc;
+  if ((rc = sim_alloc(h, &q, 8 * sizeof(int)))) return rc;
   U.cnt = (int*)q;
   CK(h, cudaMemset(U.cnt, 0, 8 * sizeof(int)));
   CK(h, cudaDeviceSynchronize());  // the legacy stream's memset, before any stream's launches
@@ -1392,9 +1448,27 @@ int enqueue_split_launch(BdHandle* h, int K, cudaStream_t s, int cur) {
 
 int build_graphs(BdHandle* h, int K) {
   const int G = launch_group(h);
-  if (h->graph_K == K && h->graph_G == G && h->graph_B == h->block && h->graph_prec == h->sp.precision &&
-      h->graph_torque == h->sp.torque_mode)
-    return BD_OK;
+  const bool split = !h->sur && G == BD_GROUP_SPLIT;
+  if (split) {
+    int rc = ensure_split_buffers(h);
+    if (rc) return rc;
+  }
+  // a graph holds its kernels and their parameters: it is good for as long as all of these are equal,
+  // byte for byte (capturing 64 split steps twice takes 6-13 ms).  The surrogate's step also depends
+  // on the ensemble's own buffers and is captured for every configuration.
+  std::vector<unsigned char> key;
+  auto add = [&](const void* v, size_t n) {
+    key.insert(key.end(), (const unsigned char*)v, (const unsigned char*)v + n);
+  };
+  const int shape[5] = {K, G, h->block, h->sp.precision, h->sp.torque_mode};
+  add(shape, sizeof shape);
+  add(&h->S, sizeof h->S);
+  add(&h->P, sizeof h->P);
+  add(h->buf, sizeof h->buf);
+  add(&h->split_buf, sizeof h->split_buf);
+  add(&h->d_live, sizeof h->d_live);
+  if (h->graph[0] && h->graph[1] && key == h->graph_key && (!h->sur || h->sur_cap == h->buf[0].cap)) return BD_OK;
+  h->graph_key.clear();
   for (auto& g : h->graph)
     if (g) {
       cudaGraphExecDestroy(g);
@@ -1406,11 +1480,6 @@ int build_graphs(BdHandle* h, int K) {
   const int sblocks = h->sur ? surrogate_blocks(h) : 0;
   if (h->sur) {
     int rc = ensure_surrogate_buffers(h);
-    if (rc) return rc;
-  }
-  const bool split = !h->sur && G == BD_GROUP_SPLIT;
-  if (split) {
-    int rc = ensure_split_buffers(h);
     if (rc) return rc;
   }
   for (int c = 0; c < 2; ++c) {
@@ -1426,11 +1495,7 @@ int build_graphs(BdHandle* h, int K) {
     cudaGraphDestroy(graph);
     CK(h, e);
   }
-  h->graph_K = K;
-  h->graph_G = G;
-  h->graph_B = h->block;
-  h->graph_prec = h->sp.precision;
-  h->graph_torque = h->sp.torque_mode;
+  h->graph_key = key;
   return BD_OK;
 }
 
@@ -1441,7 +1506,7 @@ int bd_sim_run(BdHandle* h, int n_launch, int K, void* stream) {
   if (!h) return BD_ERR_ARG;
   if (!h->sim_ready) return fail(h, BD_ERR_STATE, "bd_sim_run before bd_sim_configure");
   if (n_launch < 0 || K <= 0) return fail(h, BD_ERR_ARG, "bd_sim_run: n_launch >= 0 and steps > 0 needed");
-  if (h->dirty) return fail(h, BD_ERR_STATE, "system changed after bd_sim_reset; reset again");
+  if (h->dirty || h->rx_dirty) return fail(h, BD_ERR_STATE, "system changed after bd_sim_reset; reset again");
   if (h->sur && h->P.stats) return fail(h, BD_ERR_STATE, "per-step statistics are not collected by the surrogate stepper");
   int rc = build_graphs(h, K);
   if (rc) return rc;
@@ -1704,7 +1769,7 @@ int bd_internal_run_noalloc(BdHandle* h, const BdSimParams* p, unsigned char* sc
   if (p->slots > max_slots)
     return fail(h, BD_ERR_ARG, "bd_sim_run_noalloc: %d slots requested, the static scratch holds at most %d",
                 p->slots, max_slots);
-  if (h->dirty)
+  if (h->dirty || h->rx_dirty)
     return fail(h, BD_ERR_STATE,
                 "bd_sim_run_noalloc: the system is not on the device yet; its upload allocates, so call "
                 "bd_sim_configure or an evaluation once before");
@@ -1885,7 +1950,7 @@ int bd_multi_create(BdHandle* const* handles, int n, BdMulti** out) {
   std::vector<long long> base(n + 1, 0);
   for (int i = 0; i < n; ++i) {
     BdHandle* h = handles[i];
-    if (!h || !h->sim_ready || h->dirty)
+    if (!h || !h->sim_ready || h->dirty || h->rx_dirty)
       return bail(mfail(m, BD_ERR_STATE, "handle %d is not configured (bd_sim_configure after its last change)", i));
     if (h->device != m->device) return bail(mfail(m, BD_ERR_ARG, "handle %d is on another device", i));
     if (i == 0) {

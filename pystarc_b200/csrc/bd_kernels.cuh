@@ -1199,6 +1199,13 @@ __device__ __forceinline__ int group_fetch(unsigned long long* p, int lane, unsi
   return v > 0x7fffffffull ? 0x7fffffff : (int)v;
 }
 
+// Two grids of one lattice interleaved (the paired elec + Born grid).
+static __global__ void pair_kernel(const float* __restrict__ a, const float* __restrict__ b, float2* __restrict__ out,
+                                   long n) {
+  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x)
+    out[i] = make_float2(a[i], b[i]);
+}
+
 // Window copy of a grid (DevGrid::win): entry n holds nodes n .. n + 4/ch - 1 of
 // node n's z row, all `ch` channels of each, zero past the end of the row.
 static __global__ void window_kernel(const float* __restrict__ d, float4* __restrict__ w, long n_nodes, int nz, int ch) {
