@@ -328,6 +328,65 @@ __device__ void group_contact(const DevSystem& S, const double c[3], int lane, u
   }
 }
 
+// Force (and energy) on one charged ligand atom at lab position x: the finest electrostatic grid that
+// holds it or the far-field, and Born direction 1 (gpu_batch_engine.py:556-582).  False if the atom's
+// terms are switched off.
+template <typename FT, bool ENERGY>
+__device__ __forceinline__ bool ligand_atom(const DevSystem& S, double charge, const double x[3], bool t_grid,
+                                            bool t_ff, FT fa[3], FT& ea, unsigned& ng, unsigned& nf) {
+  const FT q = (FT)charge;
+  FT fa0 = 0, fa1 = 0, fa2 = 0;
+  ea = 0;
+  int gi = -1;
+  for (int k = 0; k < S.n_elec; ++k)
+    if (in_box(S.elec[k], x[0], x[1], x[2])) {
+      gi = k;
+      break;
+    }
+  const bool bin = S.has_born && in_box(S.born, x[0], x[1], x[2]);
+  const FT cb = (FT)S.alpha * q * q;
+  if (gi == 0 && bin && S.paired) {
+    if (!t_grid) return false;
+    const StencilOut<FT, 2> s = stencil<FT, 2>(S.pair, x[0], x[1], x[2]);
+    fa0 = -q * s.gx[0] - cb * s.gx[1];
+    fa1 = -q * s.gy[0] - cb * s.gy[1];
+    fa2 = -q * s.gz[0] - cb * s.gz[1];
+    if (ENERGY) ea = q * s.phi[0] + cb * s.phi[1];
+    ng += 2;
+  } else {
+    if (gi >= 0) {
+      if (t_grid) {
+        const StencilOut<FT, 1> s = stencil<FT, 1>(S.elec[gi], x[0], x[1], x[2]);
+        fa0 = -q * s.gx[0];
+        fa1 = -q * s.gy[0];
+        fa2 = -q * s.gz[0];
+        if (ENERGY) ea = q * s.phi[0];
+        ng += 1;
+      }
+    } else if (S.has_yukawa && t_ff) {
+      FT ff[3], ef;
+      farfield<FT>(S, x[0], x[1], x[2], q, ff, ef);
+      fa0 = ff[0];
+      fa1 = ff[1];
+      fa2 = ff[2];
+      if (ENERGY) ea = ef;
+      nf += 1;
+    }
+    if (bin && t_grid) {
+      const StencilOut<FT, 1> s = stencil<FT, 1>(S.born, x[0], x[1], x[2]);
+      fa0 -= cb * s.gx[0];
+      fa1 -= cb * s.gy[0];
+      fa2 -= cb * s.gz[0];
+      if (ENERGY) ea += cb * s.phi[0];
+      ng += 1;
+    }
+  }
+  fa[0] = fa0;
+  fa[1] = fa1;
+  fa[2] = fa2;
+  return true;
+}
+
 // Net force, torque (about c) and energy on the ligand of one trajectory,
 // computed cooperatively by the G lanes of a group.  Follows
 // GPUBatchForceEngine.__call__ (pystarc/forces/gpu_batch_engine.py:531-605):
@@ -350,60 +409,16 @@ __device__ void group_forces(const DevSystem& S, const double c[3], const double
     if (fabs(a.w) < 1e-9) continue;
     double ro[3], x[3];
     pos(i, a, ro, x);
-    const FT q = (FT)a.w;
-    FT fa0 = 0, fa1 = 0, fa2 = 0, ea = 0;
-    int gi = -1;
-    for (int k = 0; k < S.n_elec; ++k)
-      if (in_box(S.elec[k], x[0], x[1], x[2])) {
-        gi = k;
-        break;
-      }
-    const bool bin = S.has_born && in_box(S.born, x[0], x[1], x[2]);
-    const FT cb = (FT)S.alpha * q * q;
-    if (gi == 0 && bin && S.paired) {
-      if (!t_grid) continue;
-      const StencilOut<FT, 2> s = stencil<FT, 2>(S.pair, x[0], x[1], x[2]);
-      fa0 = -q * s.gx[0] - cb * s.gx[1];
-      fa1 = -q * s.gy[0] - cb * s.gy[1];
-      fa2 = -q * s.gz[0] - cb * s.gz[1];
-      if (ENERGY) ea = q * s.phi[0] + cb * s.phi[1];
-      ng += 2;
-    } else {
-      if (gi >= 0) {
-        if (t_grid) {
-        const StencilOut<FT, 1> s = stencil<FT, 1>(S.elec[gi], x[0], x[1], x[2]);
-        fa0 = -q * s.gx[0];
-        fa1 = -q * s.gy[0];
-        fa2 = -q * s.gz[0];
-        if (ENERGY) ea = q * s.phi[0];
-        ng += 1;
-        }
-      } else if (S.has_yukawa && t_ff) {
-        FT ff[3], ef;
-        farfield<FT>(S, x[0], x[1], x[2], q, ff, ef);
-        fa0 = ff[0];
-        fa1 = ff[1];
-        fa2 = ff[2];
-        if (ENERGY) ea = ef;
-        nf += 1;
-      }
-      if (bin && t_grid) {
-        const StencilOut<FT, 1> s = stencil<FT, 1>(S.born, x[0], x[1], x[2]);
-        fa0 -= cb * s.gx[0];
-        fa1 -= cb * s.gy[0];
-        fa2 -= cb * s.gz[0];
-        if (ENERGY) ea += cb * s.phi[0];
-        ng += 1;
-      }
-    }
-    f0 += (double)fa0;
-    f1 += (double)fa1;
-    f2 += (double)fa2;
+    FT fa[3], ea;
+    if (!ligand_atom<FT, ENERGY>(S, a.w, x, t_grid, t_ff, fa, ea, ng, nf)) continue;
+    f0 += (double)fa[0];
+    f1 += (double)fa[1];
+    f2 += (double)fa[2];
     if (ENERGY) e += (double)ea;
     if (TORQUE) {
-      t0 += ro[1] * (double)fa2 - ro[2] * (double)fa1;
-      t1 += ro[2] * (double)fa0 - ro[0] * (double)fa2;
-      t2 += ro[0] * (double)fa1 - ro[1] * (double)fa0;
+      t0 += ro[1] * (double)fa[2] - ro[2] * (double)fa[1];
+      t1 += ro[2] * (double)fa[0] - ro[0] * (double)fa[2];
+      t2 += ro[0] * (double)fa[1] - ro[1] * (double)fa[0];
     }
   }
   // WCA contact forces, for centroids within the activation radius (gpu_batch_engine.py:488-490)

@@ -52,6 +52,8 @@ struct OneTab {
   __device__ __forceinline__ const DevSim& sim(int) const { return P; }
   __device__ __forceinline__ int locate(int&) const { return 0; }  // trajectory id -> system, local id
   __device__ __forceinline__ int global_id(int, int id) const { return id; }
+  // every ligand has at most 32 atoms and no contact forces (which a whole warp evaluates)
+  __device__ __forceinline__ bool small_ligands() const { return S.n_lig <= 32 && !S.wca; }
   __device__ __forceinline__ void refill(Traj& tr, int&, bool& dead, int lane) const { warp_refill(P, tr, dead, lane); }
   __device__ __forceinline__ bool overlap(int, const double cn[3], bool need, int lane, const RecView& v) const {
     return warp_overlap(S, cn, need, lane, v);
@@ -211,35 +213,130 @@ __device__ __forceinline__ int next_item(int* cursor, int n_warps, int lane) {
   return __shfl_sync(0xffffffffu, j, 0);
 }
 
-// Forces on the ligand atoms of the listed poses, one warp per pose.
+// The pose of a slot: centre and rotation.  The rotation is left as a set of values, as the fused
+// stepper has it: otherwise the compiler may fuse its arithmetic with the atoms' and round the
+// positions differently.
+struct SlotPose {
+  double c[3], R[9];
+  __device__ __forceinline__ SlotPose(const SlotBuf& B, int slot) {
+    const double q[4] = {B.q[slot], B.q[B.cap + slot], B.q[2 * B.cap + slot], B.q[3 * B.cap + slot]};
+#pragma unroll
+    for (int i = 0; i < 3; ++i) c[i] = B.c[i * B.cap + slot];
+    quat_to_rot(q, R);
+#pragma unroll
+    for (int i = 0; i < 9; ++i) asm volatile("" : "+d"(R[i]));
+  }
+};
+
+// Lane i of 8 or 32 stores component i of the six.
+__device__ __forceinline__ void store_force(const SplitBuf& U, int slot, int i, const double f[3], const double t[3]) {
+  const double v = i == 0 ? f[0] : i == 1 ? f[1] : i == 2 ? f[2] : i == 3 ? t[0] : i == 4 ? t[1] : t[2];
+  if (i < 3) U.F[3 * slot + i] = v;
+  else if (i < 6) U.T[3 * slot + i - 3] = v;
+}
+
+// Forces on the ligand atoms of a pose for ligands of at most 32 atoms, by 8 lanes: lane l takes atoms
+// l, l + 8, l + 16, l + 24.  Four poses share a warp, so an 18-atom ligand fills 18 of 24 lane turns
+// instead of 18 of 32, and three reduction levels serve four poses.  The sums follow the tree of a
+// whole warp with one atom per lane (levels 16 and 8 in the lane, 4, 2, 1 across): the same bits.
+template <typename FT, bool TORQUE>
+__device__ __forceinline__ void quarter_forces(const DevSystem& S, const double c[3], const double R[9], int l,
+                                               double f[3], double t[3], Counts& cnt) {
+  const PosFromPose pos{R, c};
+  double even[3] = {0, 0, 0}, even_t[3] = {0, 0, 0}, t0 = 0, t1 = 0, t2 = 0;
+  f[0] = f[1] = f[2] = 0.0;
+#pragma unroll 1
+  for (int k = 0; k < 4; ++k) {  // turns 0, 2, then 1, 3
+    if (k == 2) {
+#pragma unroll
+      for (int d = 0; d < 3; ++d) {
+        even[d] = f[d];
+        f[d] = 0.0;
+      }
+      even_t[0] = t0;
+      even_t[1] = t1;
+      even_t[2] = t2;
+      t0 = t1 = t2 = 0.0;
+    }
+    const int i = l + 8 * (k < 2 ? 2 * k : 2 * k - 3);
+    if (i >= S.n_lig) continue;
+    const double4 a = S.lig[i];
+    if (fabs(a.w) < 1e-9) continue;
+    double ro[3], x[3];
+    pos(i, a, ro, x);
+    FT fa[3], ea;
+    if (!ligand_atom<FT, false>(S, a.w, x, true, true, fa, ea, cnt.grid, cnt.ff)) continue;
+    f[0] += (double)fa[0];
+    f[1] += (double)fa[1];
+    f[2] += (double)fa[2];
+    if (TORQUE) {
+      t0 += ro[1] * (double)fa[2] - ro[2] * (double)fa[1];
+      t1 += ro[2] * (double)fa[0] - ro[0] * (double)fa[2];
+      t2 += ro[0] * (double)fa[1] - ro[1] * (double)fa[0];
+    }
+  }
+  t[0] = t0;
+  t[1] = t1;
+  t[2] = t2;
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    f[d] = even[d] + f[d];
+    if (TORQUE) t[d] = even_t[d] + t[d];
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) {
+      f[d] += __shfl_xor_sync(0xffffffffu, f[d], o);
+      if (TORQUE) t[d] += __shfl_xor_sync(0xffffffffu, t[d], o);
+    }
+  }
+}
+
+// Forces on the ligand atoms of the listed poses: a warp per pose, or four poses per warp for small
+// ligands in mixed precision and lists of several poses a warp (18 atoms, 150,000 slots: 155 -> 116 us;
+// at 8,000 slots a warp per pose is the faster, 15.5 against 17.4 us, and in FP64 the quarter-warp
+// form spills and is slower at 30,011).  Bound by latency at 13 warps per SM: issue slots 45 %, L1 43 %,
+// the double-float conversions 22 %.
 template <typename FT, bool TORQUE, class TAB>
 __global__ void __launch_bounds__(256, 2) split_fwd_kernel(const __grid_constant__ TAB T, SlotBuf B, SplitBuf U,
                                                            int set) {
   const unsigned FULL = 0xffffffffu;
   const int lane = threadIdx.x & 31;
   const int n = U.cnt[4 * set], n_warps = (gridDim.x * blockDim.x) >> 5;
+  const int first = (threadIdx.x >> 5) * gridDim.x + blockIdx.x;
   Counts cnt{0, 0, 0};
-  for (int j = (threadIdx.x >> 5) * gridDim.x + blockIdx.x; j < n;
-       j = next_item(U.cnt + 4 * set + 2, n_warps, lane)) {
-    const int slot = U.flist[j];
-    int id = B.traj[slot];
-    const DevSystem& S = T.sys(T.locate(id));
-    const double q[4] = {B.q[slot], B.q[B.cap + slot], B.q[2 * B.cap + slot], B.q[3 * B.cap + slot]};
-    const double c[3] = {B.c[slot], B.c[B.cap + slot], B.c[2 * B.cap + slot]};
-    double R[9], f[3], t[3], e;
-    quat_to_rot(q, R);
-    // the rotation as the fused stepper has it, a set of values: without this the compiler may fuse
-    // its arithmetic with the atoms' and round the positions otherwise
+  if (sizeof(FT) == 4 && T.small_ligands() && n > 4 * n_warps) {
+    // lanes read the poses of `m` list entries together, then hand them out four at a time
+    const int m = min(32, 4 * ((n + 4 * n_warps - 1) / (4 * n_warps)));
+    for (long long base = (long long)first * m; base < n; base += (long long)n_warps * m) {
+      const int j = (int)base + lane;
+      const bool have = lane < m && j < n;
+      const int slot = have ? U.flist[j] : U.flist[(int)base];
+      const SlotPose pose(B, slot);
+      int id = B.traj[slot];
+      const int sys = T.locate(id);
+      for (int p = 0; p < m && base + p < n; p += 4) {
+        const int src = p + (lane >> 3);
+        double c[3], R[9], f[3], t[3];
 #pragma unroll
-    for (int i = 0; i < 9; ++i) asm volatile("" : "+d"(R[i]));
-    group_forces<FT, 32, TORQUE, false, PosFromPose, false>(S, c, R, lane, FULL, PosFromPose{R, c}, f, t, e, cnt,
-                                                           RecView{nullptr, nullptr});
-    if (lane == 0) {
+        for (int i = 0; i < 3; ++i) c[i] = __shfl_sync(FULL, pose.c[i], src);
 #pragma unroll
-      for (int i = 0; i < 3; ++i) {
-        U.F[3 * slot + i] = f[i];
-        U.T[3 * slot + i] = t[i];
+        for (int i = 0; i < 9; ++i) R[i] = __shfl_sync(FULL, pose.R[i], src);
+        const int to = __shfl_sync(FULL, slot, src);
+        const DevSystem& S = T.sys(__shfl_sync(FULL, sys, src));
+        quarter_forces<FT, TORQUE>(S, c, R, lane & 7, f, t, cnt);
+        if (base + src < n) store_force(U, to, lane & 7, f, t);
       }
+    }
+  } else {
+    for (int j = first; j < n; j = next_item(U.cnt + 4 * set + 2, n_warps, lane)) {
+      const int slot = U.flist[j];
+      int id = B.traj[slot];
+      const DevSystem& S = T.sys(T.locate(id));
+      const SlotPose pose(B, slot);
+      double f[3], t[3], e;
+      group_forces<FT, 32, TORQUE, false, PosFromPose, false>(S, pose.c, pose.R, lane, FULL,
+                                                             PosFromPose{pose.R, pose.c}, f, t, e, cnt,
+                                                             RecView{nullptr, nullptr});
+      store_force(U, slot, lane, f, t);
     }
   }
   const unsigned ng = gsumu<32>(cnt.grid, FULL), nf = gsumu<32>(cnt.ff, FULL);
