@@ -1377,29 +1377,38 @@ int surrogate_blocks(BdHandle* h) {
   return persistent_blocks(h, table_for(h->sp.precision, h->sp.torque_mode).sur_begin, 256);
 }
 
-// Scratch of the split stepper for the configured capacity (outside any capture).
+// Scratch of the split stepper for C slots from `alloc(void**, bytes)`.
+extern "C++" {
+template <class Alloc>
+int split_buffers(SplitBuf& U, size_t C, Alloc alloc) {
+  void* q;
+  int rc;
+  if ((rc = alloc(&q, 3 * C * sizeof(double)))) return rc;
+  U.F = (double*)q;
+  if ((rc = alloc(&q, 3 * C * sizeof(double)))) return rc;
+  U.T = (double*)q;
+  if ((rc = alloc(&q, 6 * C * sizeof(double)))) return rc;
+  U.rv = (double*)q;
+  if ((rc = alloc(&q, C * sizeof(double)))) return rc;
+  U.rprev = (double*)q;
+  if ((rc = alloc(&q, C))) return rc;
+  U.mode = (int8_t*)q;
+  if ((rc = alloc(&q, C * sizeof(int)))) return rc;
+  U.flist = (int*)q;
+  if ((rc = alloc(&q, C * sizeof(int)))) return rc;
+  U.rlist = (int*)q;
+  if ((rc = alloc(&q, 8 * sizeof(int)))) return rc;
+  U.cnt = (int*)q;
+  return BD_OK;
+}
+}  // extern "C++"
+
+// The handle's, for the configured capacity (outside any capture).
 int ensure_split_buffers(BdHandle* h) {
   const int C = h->buf[0].cap;
   if (h->split_cap == C) return BD_OK;
   SplitBuf& U = h->split_buf;
-  void* q;
-  int rc;
-  if ((rc = sim_alloc(h, &q, 3 * (size_t)C * sizeof(double)))) return rc;
-  U.F = (double*)q;
-  if ((rc = sim_alloc(h, &q, 3 * (size_t)C * sizeof(double)))) return rc;
-  U.T = (double*)q;
-  if ((rc = sim_alloc(h, &q, 6 * (size_t)C * sizeof(double)))) return rc;
-  U.rv = (double*)q;
-  if ((rc = sim_alloc(h, &q, (size_t)C * sizeof(double)))) return rc;
-  U.rprev = (double*)q;
-  if ((rc = sim_alloc(h, &q, (size_t)C))) return rc;
-  U.mode = (int8_t*)q;
-  if ((rc = sim_alloc(h, &q, (size_t)C * sizeof(int)))) return rc;
-  U.flist = (int*)q;
-  if ((rc = sim_alloc(h, &q, (size_t)C * sizeof(int)))) return rc;
-  U.rlist = (int*)q;
-  if ((rc = sim_alloc(h, &q, 8 * sizeof(int)))) return rc;
-  U.cnt = (int*)q;
+  if (int rc = split_buffers(U, (size_t)C, [&](void** q, size_t b) { return sim_alloc(h, q, b); })) return rc;
   CK(h, cudaMemset(U.cnt, 0, 8 * sizeof(int)));
   CK(h, cudaDeviceSynchronize());  // the legacy stream's memset, before any stream's launches
   if (!h->side) CK(h, cudaStreamCreateWithFlags(&h->side, cudaStreamNonBlocking));
@@ -1409,40 +1418,62 @@ int ensure_split_buffers(BdHandle* h) {
   return BD_OK;
 }
 
-// K split steps on buffer `cur`, then the compaction into the other buffer.  The two force
-// kernels of a step do not depend on each other: the sweep is captured on a branch of its own.
-int enqueue_split_launch(BdHandle* h, int K, cudaStream_t s, int cur) {
-  const SplitKernels& kn = table_for(h->sp.precision, h->sp.torque_mode).split;
-  const size_t smem = stepper_smem(h->S, h->P, kn.mid);
-  stepper_smem(h->S, h->P, kn.last);
-  const int b_step = persistent_blocks(h, kn.mid, kStepBlock, smem), b_fwd = persistent_blocks(h, kn.fwd, 256),
-            b_rev = persistent_blocks(h, kn.rev, 256);
-  SlotBuf src = h->buf[cur], dst = h->buf[1 - cur];
-  const int* live = h->d_live + cur;
-  SplitBuf U = h->split_buf;
-  OneTab T{h->S, h->P};
+// K split steps on the slots of `src`, then the compaction into `dst`.  The two force kernels of a
+// step do not depend on each other: the sweep is captured on a branch of its own.
+struct SplitPlan {
+  const SplitKernels* kn;
+  void* tab;       // OneTab or MultiTab (copied at capture)
+  SplitBuf U;
+  bool rev;        // some system has Born direction 2
+  size_t smem;     // of the scalar kernel when it ends a step
+  int b_step, b_fwd, b_rev;
+  cudaStream_t side;
+  cudaEvent_t fork, join;
+  unsigned long long* ctr;
+  int n_sm;
+};
+
+cudaError_t enqueue_split_steps(const SplitPlan& p, SlotBuf src, SlotBuf dst, const int* live, int* live_dst, int K,
+                                cudaStream_t s) {
+  SplitBuf U = p.U;
+  cudaError_t e = cudaSuccess;
+  auto ok = [&](cudaError_t x) { return (e = x) == cudaSuccess; };
   for (int k = 0; k <= K; ++k) {
     int set = k & 1;
-    void* s_args[] = {&T, &src, &live, &U, &set};
-    if (k == K) {
-      CK(h, cudaLaunchKernel(kn.last, dim3(b_step), dim3(kStepBlock), s_args, smem, s));
-      break;
+    void* s_args[] = {p.tab, &src, &live, &U, &set};
+    void* fn = k == 0 ? p.kn->first : k == K ? p.kn->last : p.kn->mid;
+    if (!ok(cudaLaunchKernel(fn, dim3(p.b_step), dim3(kStepBlock), s_args, k == 0 ? 0 : p.smem, s))) return e;
+    if (k == K) break;
+    void* f_args[] = {p.tab, &src, &U, &set};
+    if (p.rev) {
+      if (!ok(cudaEventRecord(p.fork, s)) || !ok(cudaStreamWaitEvent(p.side, p.fork, 0)) ||
+          !ok(cudaLaunchKernel(p.kn->rev, dim3(p.b_rev), dim3(256), f_args, 0, p.side)) ||
+          !ok(cudaEventRecord(p.join, p.side)))
+        return e;
     }
-    CK(h, cudaLaunchKernel(k == 0 ? kn.first : kn.mid, dim3(b_step), dim3(kStepBlock), s_args, k == 0 ? 0 : smem, s));
-    void* f_args[] = {&T, &src, &U, &set};
-    if (h->S.born_rev) {
-      CK(h, cudaEventRecord(h->fork, s));
-      CK(h, cudaStreamWaitEvent(h->side, h->fork, 0));
-      CK(h, cudaLaunchKernel(kn.rev, dim3(b_rev), dim3(256), f_args, 0, h->side));
-      CK(h, cudaEventRecord(h->join, h->side));
-    }
-    CK(h, cudaLaunchKernel(kn.fwd, dim3(b_fwd), dim3(256), f_args, 0, s));
-    if (h->S.born_rev) CK(h, cudaStreamWaitEvent(s, h->join, 0));
+    if (!ok(cudaLaunchKernel(p.kn->fwd, dim3(p.b_fwd), dim3(256), f_args, 0, s))) return e;
+    if (p.rev && !ok(cudaStreamWaitEvent(s, p.join, 0))) return e;
   }
-  compact_kernel<<<h->n_sm * 4, 256, 0, s>>>(src, dst, live, h->d_ctr);
-  CK(h, cudaGetLastError());
-  finish_compact_kernel<<<1, 1, 0, s>>>(h->d_live + (1 - cur), h->d_ctr);
-  CK(h, cudaGetLastError());
+  compact_kernel<<<p.n_sm * 4, 256, 0, s>>>(src, dst, live, p.ctr);
+  if (!ok(cudaGetLastError())) return e;
+  finish_compact_kernel<<<1, 1, 0, s>>>(live_dst, p.ctr);
+  return cudaGetLastError();
+}
+
+int enqueue_split_launch(BdHandle* h, int K, cudaStream_t s, int cur) {
+  const SplitKernels& kn = table_for(h->sp.precision, h->sp.torque_mode).split;
+  OneTab T{h->S, h->P};
+  SplitPlan p{&kn, &T, h->split_buf, h->S.born_rev != 0, stepper_smem(h->S, h->P, kn.mid)};
+  stepper_smem(h->S, h->P, kn.last);
+  p.b_step = persistent_blocks(h, kn.mid, kStepBlock, p.smem);
+  p.b_fwd = persistent_blocks(h, kn.fwd, 256);
+  p.b_rev = persistent_blocks(h, kn.rev, 256);
+  p.side = h->side;
+  p.fork = h->fork;
+  p.join = h->join;
+  p.ctr = h->d_ctr;
+  p.n_sm = h->n_sm;
+  CK(h, enqueue_split_steps(p, h->buf[cur], h->buf[1 - cur], h->d_live + cur, h->d_live + (1 - cur), K, s));
   return BD_OK;
 }
 
@@ -1859,9 +1890,12 @@ struct BdMulti {
   MultiTab T{};
   SlotBuf buf[2]{};
   int* d_live = nullptr;
-  int cap = 0, cur = 0, blocks = 0;
+  int cap = 0, cur = 0;
+  bool rev = false;  // some system has Born direction 2
+  SplitBuf split{};
   std::vector<void*> allocs;
-  cudaStream_t own = nullptr;
+  cudaStream_t own = nullptr, side = nullptr;
+  cudaEvent_t fork = nullptr, join = nullptr;
   cudaGraphExec_t graph[2] = {nullptr, nullptr};
   int graph_K = -1;
   std::string err;
@@ -1893,8 +1927,6 @@ int malloc_multi(BdMulti* m, void** p, size_t bytes) {
   return BD_OK;
 }
 
-void* multi_kernel(int prec, int torque) { return table_for(prec, torque).multi; }
-
 int multi_graphs(BdMulti* m, int K) {
   if (m->graph_K == K) return BD_OK;
   for (auto& g : m->graph)
@@ -1902,21 +1934,26 @@ int multi_graphs(BdMulti* m, int K) {
       cudaGraphExecDestroy(g);
       g = nullptr;
     }
-  void* fn = multi_kernel(m->precision, m->torque);
+  const SplitKernels& kn = table_for(m->precision, m->torque).multi;
+  auto blocks = [&](void* fn, int block) {
+    int per_sm = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, block, 0) != cudaSuccess || per_sm < 1) per_sm = 1;
+    return per_sm * m->n_sm;
+  };
+  MultiTab T = m->T;
+  SplitPlan p{&kn, &T, m->split, m->rev, 0};
+  p.b_step = blocks(kn.mid, kStepBlock);
+  p.b_fwd = blocks(kn.fwd, 256);
+  p.b_rev = blocks(kn.rev, 256);
+  p.side = m->side;
+  p.fork = m->fork;
+  p.join = m->join;
+  p.ctr = m->T.ctr;
+  p.n_sm = m->n_sm;
   for (int c = 0; c < 2; ++c) {
     cudaGraph_t graph;
     MCK(m, cudaStreamBeginCapture(m->own, cudaStreamCaptureModeThreadLocal));
-    SlotBuf src = m->buf[c], dst = m->buf[1 - c];
-    const int* live = m->d_live + c;
-    int KK = K;
-    MultiTab T = m->T;
-    void* args[] = {&T, &src, &live, &KK};
-    cudaError_t e = cudaLaunchKernel(fn, dim3(m->blocks), dim3(256), args, 0, m->own);
-    if (e == cudaSuccess) {
-      compact_kernel<<<m->n_sm * 4, 256, 0, m->own>>>(src, dst, live, m->T.ctr);
-      finish_compact_kernel<<<1, 1, 0, m->own>>>(m->d_live + (1 - c), m->T.ctr);
-      e = cudaGetLastError();
-    }
+    cudaError_t e = enqueue_split_steps(p, m->buf[c], m->buf[1 - c], m->d_live + c, m->d_live + (1 - c), K, m->own);
     cudaError_t e2 = cudaStreamEndCapture(m->own, &graph);
     MCK(m, e);
     MCK(m, e2);
@@ -1939,6 +1976,9 @@ int bd_multi_create(BdHandle* const* handles, int n, BdMulti** out) {
   BdMulti* m = new BdMulti();
   auto bail = [&](int rc) {
     for (void* p : m->allocs) cudaFree(p);
+    if (m->fork) cudaEventDestroy(m->fork);
+    if (m->join) cudaEventDestroy(m->join);
+    if (m->side) cudaStreamDestroy(m->side);
     if (m->own) cudaStreamDestroy(m->own);
     g_create_error = m->err;
     delete m;
@@ -1965,6 +2005,8 @@ int bd_multi_create(BdHandle* const* handles, int n, BdMulti** out) {
     sim[i] = h->P;
     sim[i].stats = 0;
     base[i + 1] = base[i] + h->P.n_traj;
+    m->rev = m->rev || h->S.born_rev;
+    m->T.small = (i == 0 || m->T.small) && h->S.n_lig <= 32 && !h->S.wca;
   }
   if (base[n] > 0x7fffffffll) return bail(mfail(m, BD_ERR_ARG, "more than 2^31 - 1 trajectories in the batch"));
   if (cudaSetDevice(m->device) != cudaSuccess) return bail(mfail(m, BD_ERR_CUDA, "cudaSetDevice failed"));
@@ -1977,11 +2019,11 @@ int bd_multi_create(BdHandle* const* handles, int n, BdMulti** out) {
   if ((rc = malloc_multi(m, &p, n * sizeof(DevSystem)))) return bail(rc);
   if (cudaMemcpy(p, sys.data(), n * sizeof(DevSystem), cudaMemcpyHostToDevice) != cudaSuccess)
     return bail(mfail(m, BD_ERR_CUDA, "upload of the system table failed"));
-  m->T.sys = (const DevSystem*)p;
+  m->T.sys_ = (const DevSystem*)p;
   if ((rc = malloc_multi(m, &p, n * sizeof(DevSim)))) return bail(rc);
   if (cudaMemcpy(p, sim.data(), n * sizeof(DevSim), cudaMemcpyHostToDevice) != cudaSuccess)
     return bail(mfail(m, BD_ERR_CUDA, "upload of the run-parameter table failed"));
-  m->T.sim = (const DevSim*)p;
+  m->T.sim_ = (const DevSim*)p;
   if ((rc = malloc_multi(m, &p, (n + 1) * sizeof(long long)))) return bail(rc);
   if (cudaMemcpy(p, base.data(), (n + 1) * sizeof(long long), cudaMemcpyHostToDevice) != cudaSuccess)
     return bail(mfail(m, BD_ERR_CUDA, "upload of the index table failed"));
@@ -1990,12 +2032,8 @@ int bd_multi_create(BdHandle* const* handles, int n, BdMulti** out) {
   m->T.total = base[n];
   m->T.ctr = ctr;
   m->hs.assign(handles, handles + n);
-  // slot pool: eight resident waves, at least 65536, at most every trajectory
-  void* fn = multi_kernel(m->precision, m->torque);
-  int per_sm = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, 256, 0) != cudaSuccess || per_sm < 1) per_sm = 1;
-  m->blocks = per_sm * m->n_sm;
-  const long long cap = std::min<long long>(base[n], std::max<long long>(65536, 8ll * m->blocks * 256));
+  // slot pool: eight waves of two 256-thread blocks per SM, at least 65536, at most every trajectory
+  const long long cap = std::min<long long>(base[n], std::max<long long>(65536, 8ll * 2 * m->n_sm * 256));
   m->cap = (int)cap;
   for (int b = 0; b < 2; ++b) {
     SlotBuf& B = m->buf[b];
@@ -2017,7 +2055,14 @@ int bd_multi_create(BdHandle* const* handles, int n, BdMulti** out) {
   }
   if ((rc = malloc_multi(m, &p, 2 * sizeof(int)))) return bail(rc);
   m->d_live = (int*)p;
-  if (cudaStreamCreateWithFlags(&m->own, cudaStreamNonBlocking) != cudaSuccess)
+  if ((rc = split_buffers(m->split, (int)cap, [&](void** q, size_t b) { return malloc_multi(m, q, b); })))
+    return bail(rc);
+  if (cudaMemset(m->split.cnt, 0, 8 * sizeof(int)) != cudaSuccess || cudaDeviceSynchronize() != cudaSuccess)
+    return bail(mfail(m, BD_ERR_CUDA, "clearing the list counters failed"));
+  if (cudaStreamCreateWithFlags(&m->own, cudaStreamNonBlocking) != cudaSuccess ||
+      cudaStreamCreateWithFlags(&m->side, cudaStreamNonBlocking) != cudaSuccess ||
+      cudaEventCreateWithFlags(&m->fork, cudaEventDisableTiming) != cudaSuccess ||
+      cudaEventCreateWithFlags(&m->join, cudaEventDisableTiming) != cudaSuccess)
     return bail(mfail(m, BD_ERR_CUDA, "stream creation failed"));
   *out = m;
   return BD_OK;
@@ -2030,6 +2075,9 @@ int bd_multi_destroy(BdMulti* m) {
   for (auto& g : m->graph)
     if (g) cudaGraphExecDestroy(g);
   for (void* p : m->allocs) cudaFree(p);
+  if (m->fork) cudaEventDestroy(m->fork);
+  if (m->join) cudaEventDestroy(m->join);
+  if (m->side) cudaStreamDestroy(m->side);
   if (m->own) cudaStreamDestroy(m->own);
   delete m;
   return BD_OK;

@@ -20,9 +20,8 @@ struct SplitKernels {
 struct KernelTable {
   void *pose[5], *atoms[5], *step[5];  // by kGroups
   void *warp, *warp_capped;            // step_kernel_warp without a register cap and at 128
-  void* multi;
   void *sur_begin, *sur_end;
-  SplitKernels split;
+  SplitKernels split, multi;           // of one system, of a heterogeneous batch
 };
 
 template <typename FT, bool TQ, class TAB>
@@ -43,10 +42,10 @@ KernelTable make_table() {
            (void*)&step_kernel<FT, 16, TQ>, (void*)&step_kernel<FT, 32, TQ>},
           (void*)&step_kernel_warp<FT, TQ, 1>,
           (void*)&step_kernel_warp<FT, TQ, 2>,
-          (void*)&step_kernel_multi<FT, TQ>,
           (void*)&sur_begin_kernel<FT, TQ>,
           (void*)&sur_end_kernel<FT, TQ>,
-          split_kernels<FT, TQ, OneTab>()};
+          split_kernels<FT, TQ, OneTab>(),
+          split_kernels<FT, TQ, MultiTab>()};
 }
 
 KernelTable table_mixed();
