@@ -2007,6 +2007,7 @@ int bd_multi_create(BdHandle* const* handles, int n, BdMulti** out) {
     base[i + 1] = base[i] + h->P.n_traj;
     m->rev = m->rev || h->S.born_rev;
     m->T.small = (i == 0 || m->T.small) && h->S.n_lig <= 32 && !h->S.wca;
+    m->T.large = (i == 0 || m->T.large) && h->S.n_lig >= 128 && !h->S.wca;
   }
   if (base[n] > 0x7fffffffll) return bail(mfail(m, BD_ERR_ARG, "more than 2^31 - 1 trajectories in the batch"));
   if (cudaSetDevice(m->device) != cudaSuccess) return bail(mfail(m, BD_ERR_CUDA, "cudaSetDevice failed"));

@@ -44,6 +44,18 @@ struct SplitBuf {
                    // turn: a step's scalar kernel fills one set and clears the other
 };
 
+// Where a force kernel reads a pose: here a slot of the stepper's pool.
+struct SlotSrc {
+  const SlotBuf& B;
+  int slot;
+  __device__ __forceinline__ void load(double c[3], double R[9]) const {
+    const double q[4] = {B.q[slot], B.q[B.cap + slot], B.q[2 * B.cap + slot], B.q[3 * B.cap + slot]};
+#pragma unroll
+    for (int i = 0; i < 3; ++i) c[i] = B.c[i * B.cap + slot];
+    quat_to_rot(q, R);
+  }
+};
+
 // One receptor-ligand system for all slots.
 struct OneTab {
   DevSystem S;
@@ -54,6 +66,8 @@ struct OneTab {
   __device__ __forceinline__ int global_id(int, int id) const { return id; }
   // every ligand has at most 32 atoms and no contact forces (which a whole warp evaluates)
   __device__ __forceinline__ bool small_ligands() const { return S.n_lig <= 32 && !S.wca; }
+  // ligands worth sharing among warps: every one of at least 128 atoms, no contact forces
+  __device__ __forceinline__ bool large_ligands() const { return S.n_lig >= 128 && !S.wca; }
   __device__ __forceinline__ void refill(Traj& tr, int&, bool& dead, int lane) const { warp_refill(P, tr, dead, lane); }
   __device__ __forceinline__ bool overlap(int, const double cn[3], bool need, int lane, const RecView& v) const {
     return warp_overlap(S, cn, need, lane, v);
@@ -213,16 +227,14 @@ __device__ __forceinline__ int next_item(int* cursor, int n_warps, int lane) {
   return __shfl_sync(0xffffffffu, j, 0);
 }
 
-// The pose of a slot: centre and rotation.  The rotation is left as a set of values, as the fused
+// The pose of a source: centre and rotation.  The rotation is left as a set of values, as the fused
 // stepper has it: otherwise the compiler may fuse its arithmetic with the atoms' and round the
 // positions differently.
-struct SlotPose {
+template <class SRC>
+struct Pose {
   double c[3], R[9];
-  __device__ __forceinline__ SlotPose(const SlotBuf& B, int slot) {
-    const double q[4] = {B.q[slot], B.q[B.cap + slot], B.q[2 * B.cap + slot], B.q[3 * B.cap + slot]};
-#pragma unroll
-    for (int i = 0; i < 3; ++i) c[i] = B.c[i * B.cap + slot];
-    quat_to_rot(q, R);
+  __device__ __forceinline__ explicit Pose(const SRC& src) {
+    src.load(c, R);
 #pragma unroll
     for (int i = 0; i < 9; ++i) asm volatile("" : "+d"(R[i]));
   }
@@ -290,6 +302,79 @@ __device__ __forceinline__ void quarter_forces(const DevSystem& S, const double 
   }
 }
 
+// A product rounded by itself: never fused into the sum it goes to.
+__device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
+
+// Barrier of the `threads` threads of a block that share named barrier `id`.
+__device__ __forceinline__ void group_sync(int id, int threads) {
+  asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
+
+// Forces on the ligand atoms of a pose by W = 2, 4 or 8 warps of a block: in a round, warp w takes the
+// 32 atoms after those of warp w - 1 and leaves every lane's terms in shared memory (`sh`: two rounds of
+// W rows of NC components of 32 lanes); component k is then summed by warp k mod W, lane by lane in the
+// order of the atoms, as a single warp sums them: the same bits.  tot[i] receives component gw + i * W
+// (f0..f2, t0..t2 with TORQUE, the energy last with ENERGY), reduced over the lanes.  Contact forces are
+// not included.
+template <bool TORQUE, bool ENERGY>
+constexpr int kForwardNc = 3 + (TORQUE ? 3 : 0) + (ENERGY ? 1 : 0);
+
+template <typename FT, bool TORQUE, bool ENERGY, class PosFn>
+__device__ __forceinline__ void group_forward(const DevSystem& S, const PosFn& pos, int lane, int gw, int W, int bar,
+                                              double* sh, bool t_grid, bool t_ff, double tot[4], Counts& cnt) {
+  constexpr int NC = kForwardNc<TORQUE, ENERGY>;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) tot[i] = 0.0;
+  int flip = 0;
+  for (int i0 = 0; i0 < S.n_lig; i0 += 32 * W) {
+    double f[3] = {0, 0, 0}, t[3] = {0, 0, 0}, e = 0;
+    const int i = i0 + 32 * gw + lane;
+    if (i < S.n_lig) {
+      const double4 a = S.lig[i];
+      double ro[3], x[3];
+      pos(i, a, ro, x);
+      FT fa[3], ea;
+      if (fabs(a.w) >= 1e-9 && ligand_atom<FT, ENERGY>(S, a.w, x, t_grid, t_ff, fa, ea, cnt.grid, cnt.ff)) {
+#pragma unroll
+        for (int d = 0; d < 3; ++d) f[d] = (double)fa[d];
+        if (ENERGY) e = (double)ea;
+        if (TORQUE) {
+          t[0] = ro[1] * (double)fa[2] - ro[2] * (double)fa[1];
+          t[1] = ro[2] * (double)fa[0] - ro[0] * (double)fa[2];
+          t[2] = ro[0] * (double)fa[1] - ro[1] * (double)fa[0];
+        }
+      }
+    }
+    double* row = sh + ((size_t)flip * W + gw) * NC * 32 + lane;
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      row[d * 32] = f[d];
+      if (TORQUE) row[(3 + d) * 32] = t[d];
+    }
+    if (ENERGY) row[(NC - 1) * 32] = e;
+    group_sync(bar, 32 * W);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const int c = gw + k * W;
+      if (c < NC)
+        for (int w = 0; w < W; ++w) tot[k] += sh[(((size_t)flip * W + w) * NC + c) * 32 + lane];
+    }
+    flip ^= 1;
+  }
+#pragma unroll
+  for (int k = 0; k < 4; ++k)
+    if (gw + k * W < NC) tot[k] = gsum<32>(tot[k], 0xffffffffu);
+}
+
+// Warps per pose of the forward forces of a large ligand, for a list of n poses on n_warps warps: only
+// where the list leaves most warps idle.  1,401 atoms, mixed precision, 128 steps, GPU time with one
+// warp per pose -> with this rule: 100 trajectories 15.7 -> 6.5 ms, 700 18.1 -> 10.8, 2,000 22.8 -> 21.9,
+// 6,000 34.9 both (two or eight warps there: 10 % slower, the rounds' barriers).
+__device__ __forceinline__ int fwd_warps(int n, int n_warps) {
+  return n * 8 <= n_warps ? 8 : n * 4 <= n_warps ? 4 : n * 2 <= n_warps ? 2 : 1;
+}
+
 // Forces on the ligand atoms of the listed poses: a warp per pose, or four poses per warp for small
 // ligands in mixed precision and lists of several poses a warp (18 atoms, 150,000 slots: 155 -> 116 us;
 // at 8,000 slots a warp per pose is the faster, 15.5 against 17.4 us, and in FP64 the quarter-warp
@@ -310,7 +395,7 @@ __global__ void __launch_bounds__(256, 2) split_fwd_kernel(const __grid_constant
       const int j = (int)base + lane;
       const bool have = lane < m && j < n;
       const int slot = have ? U.flist[j] : U.flist[(int)base];
-      const SlotPose pose(B, slot);
+      const Pose<SlotSrc> pose(SlotSrc{B, slot});
       int id = B.traj[slot];
       const int sys = T.locate(id);
       for (int p = 0; p < m && base + p < n; p += 4) {
@@ -326,12 +411,31 @@ __global__ void __launch_bounds__(256, 2) split_fwd_kernel(const __grid_constant
         if (base + src < n) store_force(U, to, lane & 7, f, t);
       }
     }
+  } else if (const int W = T.large_ligands() ? fwd_warps(n, n_warps) : 1; W > 1) {
+    constexpr int NC = kForwardNc<TORQUE, false>;
+    __shared__ double sh[2 * 8 * NC * 32];
+    const int warp = threadIdx.x >> 5, gw = warp & (W - 1), grp = warp / W;
+    for (int j = grp * gridDim.x + blockIdx.x; j < n; j += n_warps / W) {
+      const int slot = U.flist[j];
+      int id = B.traj[slot];
+      const DevSystem& S = T.sys(T.locate(id));
+      const Pose<SlotSrc> pose(SlotSrc{B, slot});
+      double tot[4];
+      group_forward<FT, TORQUE, false>(S, PosFromPose{pose.R, pose.c}, lane, gw, W, 1 + grp, sh + 2 * grp * W * NC * 32,
+                                       true, true, tot, cnt);
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const int c = gw + k * W;
+        if (lane == 0 && c < 3) U.F[3 * slot + c] = tot[k];
+        if (lane == 0 && c >= 3 && c < 6) U.T[3 * slot + c - 3] = TORQUE ? tot[k] : 0.0;
+      }
+    }
   } else {
     for (int j = first; j < n; j = next_item(U.cnt + 4 * set + 2, n_warps, lane)) {
       const int slot = U.flist[j];
       int id = B.traj[slot];
       const DevSystem& S = T.sys(T.locate(id));
-      const SlotPose pose(B, slot);
+      const Pose<SlotSrc> pose(SlotSrc{B, slot});
       double f[3], t[3], e;
       group_forces<FT, 32, TORQUE, false, PosFromPose, false>(S, pose.c, pose.R, lane, FULL,
                                                              PosFromPose{pose.R, pose.c}, f, t, e, cnt,
@@ -345,22 +449,22 @@ __global__ void __launch_bounds__(256, 2) split_fwd_kernel(const __grid_constant
   if (lane == 0 && nf) atomicAdd(ctr + C_FF_EVALS, (unsigned long long)nf);
 }
 
-// The pose of slot `slot` as the sweep of direction 2 needs it: rotation and centre in FT, and its
+// The pose of a source as the sweep of direction 2 needs it: rotation and centre in FT, and its
 // tests of receptor chunks and atoms against the ligand Born grid's margin box in the ligand frame.
 template <typename FT>
 struct RevPose {
   using V4 = typename Vec4<FT>::type;
   FT Rt[9], cx, cy, cz;
 
-  __device__ __forceinline__ RevPose(const SlotBuf& B, int slot) {
-    const double q[4] = {B.q[slot], B.q[B.cap + slot], B.q[2 * B.cap + slot], B.q[3 * B.cap + slot]};
-    double R[9];
-    quat_to_rot(q, R);
+  template <class SRC>
+  __device__ __forceinline__ explicit RevPose(const SRC& src) {
+    double c[3], R[9];
+    src.load(c, R);
 #pragma unroll
     for (int k = 0; k < 9; ++k) Rt[k] = (FT)R[k];
-    cx = (FT)B.c[slot];
-    cy = (FT)B.c[B.cap + slot];
-    cz = (FT)B.c[2 * B.cap + slot];
+    cx = (FT)c[0];
+    cy = (FT)c[1];
+    cz = (FT)c[2];
   }
 
   // Chunk k's bounding sphere reaches the box.
@@ -384,7 +488,8 @@ struct RevPose {
   }
 
   // Receptor atom idx is charged and inside the box; e = its ligand-frame position and charge.
-  __device__ __forceinline__ bool candidate(const DevSystem& S, const SlotBuf& B, int slot, int idx, V4& e) const {
+  template <class SRC>
+  __device__ __forceinline__ bool candidate(const DevSystem& S, const SRC& src, int idx, V4& e) const {
     const DevGrid& g = S.lig_born;
     const FT lox = (FT)g.lox, loy = (FT)g.loy, loz = (FT)g.loz, hix = (FT)g.hix, hiy = (FT)g.hiy, hiz = (FT)g.hiz;
     V4 at;
@@ -400,11 +505,10 @@ struct RevPose {
       // within 1e-3 A of a face the FP64 box test decides (the set of atoms is the FP64 one)
       const float m = fminf(fminf(fminf(l0 - lox, hix - l0), fminf(l1 - loy, hiy - l1)), fminf(l2 - loz, hiz - l2));
       if (fabsf(m) < 1e-3f) {
-        const double q[4] = {B.q[slot], B.q[B.cap + slot], B.q[2 * B.cap + slot], B.q[3 * B.cap + slot]};
-        double R[9];
-        quat_to_rot(q, R);
+        double c[3], R[9];
+        src.load(c, R);
         const double4 a64 = S.rec[idx];
-        const double e0 = a64.x - B.c[slot], e1 = a64.y - B.c[B.cap + slot], e2 = a64.z - B.c[2 * B.cap + slot];
+        const double e0 = a64.x - c[0], e1 = a64.y - c[1], e2 = a64.z - c[2];
         cand = in_box(g, R[0] * e0 + R[3] * e1 + R[6] * e2, R[1] * e0 + R[4] * e1 + R[7] * e2,
                       R[2] * e0 + R[5] * e1 + R[8] * e2);
       }
@@ -418,14 +522,14 @@ struct RevPose {
 // receptor chunks culled against the ligand Born grid's margin box in the ligand frame, in-box
 // atoms gathered into `buf` and drained 32 at a time.  Adds this lane's share of the sums to
 // r (ligand frame) and u; the caller reduces over the warp.
-template <typename FT, bool TORQUE>
-__device__ __forceinline__ void lean_reverse_born(const DevSystem& S, const SlotBuf& B, int slot, int lane,
+template <typename FT, bool TORQUE, class SRC>
+__device__ __forceinline__ void lean_reverse_born(const DevSystem& S, const SRC& src, int lane,
                                                   typename Vec4<FT>::type* buf, double r[3], double u[3],
                                                   unsigned& nr) {
   using V4 = typename Vec4<FT>::type;
   const unsigned FULL = 0xffffffffu;
   const DevGrid& g = S.lig_born;
-  const RevPose<FT> pose(B, slot);
+  const RevPose<FT> pose(src);
   FT rs0 = 0, rs1 = 0, rs2 = 0;
   int k0 = 0, head = 0;
   unsigned hits = 0;
@@ -445,7 +549,7 @@ __device__ __forceinline__ void lean_reverse_born(const DevSystem& S, const Slot
       const int kk = k0 - 32 + __ffs(hits) - 1;
       hits &= hits - 1;
       V4 ent{};
-      const bool cand = pose.candidate(S, B, slot, kk * BD_CHUNK + lane, ent);
+      const bool cand = pose.candidate(S, src, kk * BD_CHUNK + lane, ent);
       const unsigned m = __ballot_sync(FULL, cand);
       if (cand) buf[head + __popc(m & ((1u << lane) - 1u))] = ent;
       head += __popc(m);
@@ -488,15 +592,6 @@ __device__ __forceinline__ void lean_reverse_born(const DevSystem& S, const Slot
   r[2] += (double)rs2;
 }
 
-// A product rounded by itself: never fused into the sum it goes to.
-__device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
-__device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
-
-// Barrier of the `threads` threads of a block that share named barrier `id`.
-__device__ __forceinline__ void group_sync(int id, int threads) {
-  asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
-}
-
 // Born direction 2 of one pose by W = 2, 4 or 8 warps of a block: warp gw of the group gathers
 // every W-th hit chunk, the entries land in `buf` (W * kSplitBuf of them) in the order of
 // lean_reverse_born, every thread evaluates stencils, and the sums are then taken entry by entry
@@ -505,15 +600,14 @@ __device__ __forceinline__ void group_sync(int id, int threads) {
 // coefficient and gradient (it is `buf` itself when the positions are not needed again);
 // cnt: two rows of W counts.  Every warp of the group takes the same path (the culls and counts
 // it depends on are the same on each), so the group's barriers match.
-template <typename FT, bool TORQUE>
-__device__ __forceinline__ void group_reverse_born(const DevSystem& S, const SlotBuf& B, int slot, int lane, int gw,
-                                                   int W, int bar, typename Vec4<FT>::type* buf,
+template <typename FT, bool TORQUE, class SRC>
+__device__ __forceinline__ void group_reverse_born(const DevSystem& S, const SRC& src, int lane, int gw, int W, int bar, typename Vec4<FT>::type* buf,
                                                    typename Vec4<FT>::type* val, int* cnt, double r[3], double u[3],
                                                    unsigned& nr) {
   using V4 = typename Vec4<FT>::type;
   const unsigned FULL = 0xffffffffu;
   const DevGrid& g = S.lig_born;
-  const RevPose<FT> pose(B, slot);
+  const RevPose<FT> pose(src);
   const FT alpha = (FT)S.alpha;
   FT rs0 = 0, rs1 = 0, rs2 = 0;
   int head = 0, flip = 0;
@@ -581,12 +675,12 @@ __device__ __forceinline__ void group_reverse_born(const DevSystem& S, const Slo
       if (h < H) {
         // the chunk of hit h: its mask's lane, then the bit with that many hits below it
         const unsigned has = __ballot_sync(FULL, before <= h && h < before + __popc(mine));
-        const int src = __ffs(has) - 1;
-        const unsigned m = __shfl_sync(FULL, mine, src);
-        const int nth = h - __shfl_sync(FULL, before, src);
+        const int ml = __ffs(has) - 1;
+        const unsigned m = __shfl_sync(FULL, mine, ml);
+        const int nth = h - __shfl_sync(FULL, before, ml);
         const unsigned at =
             __ballot_sync(FULL, ((m >> lane) & 1u) && __popc(m & ((1u << lane) - 1u)) == nth);
-        cand = pose.candidate(S, B, slot, (c0 + 32 * src + __ffs(at) - 1) * BD_CHUNK + lane, ent);
+        cand = pose.candidate(S, src, (c0 + 32 * ml + __ffs(at) - 1) * BD_CHUNK + lane, ent);
       }
       const unsigned m = __ballot_sync(FULL, cand);
       if (lane == 0) cnt[flip * 8 + gw] = __popc(m);
@@ -649,11 +743,11 @@ __global__ void __launch_bounds__(256, sizeof(FT) == 4 ? 4 : 2) split_rev_kernel
     const DevSystem& S = T.sys(T.locate(id));
     double r[3] = {0, 0, 0}, u[3] = {0, 0, 0};
     if (W == 1) {
-      lean_reverse_born<FT, TORQUE>(S, B, slot, lane, bufs[warp], r, u, nr);
+      lean_reverse_born<FT, TORQUE>(S, SlotSrc{B, slot}, lane, bufs[warp], r, u, nr);
     } else {
       V4* buf = bufs[grp * W];
-      group_reverse_born<FT, TORQUE>(S, B, slot, lane, gw, W, 1 + grp, buf, TORQUE ? vals[grp * W] : buf, cnts[grp], r,
-                                     u, nr);
+      group_reverse_born<FT, TORQUE>(S, SlotSrc{B, slot}, lane, gw, W, 1 + grp, buf, TORQUE ? vals[grp * W] : buf,
+                                     cnts[grp], r, u, nr);
     }
     if (gw == 0) {
       r[0] = gsum<32>(r[0], FULL);

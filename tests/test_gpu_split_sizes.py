@@ -32,3 +32,23 @@ def test_split_outcomes_equal_the_fused_steppers(n, slots, K, precision, sysname
     for x, y in zip(outs[0][0], outs[1][0]):
         np.testing.assert_array_equal(x, y)
     assert outs[0][1] == outs[1][1]
+
+
+@pytest.mark.parametrize("n,K", [(1, 1), (200, 3), (550, 2), (1100, 4), (2500, 2)])
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_large_ligands_shared_among_warps(n, K, precision):
+    """A 176-atom ligand (ragged against 32 atoms a warp and a round): eight, four, two warps and one per pose."""
+    from pystarc_b200 import synth
+
+    s = synth.config3(scale=0.5, device="cuda")
+    outs = []
+    for group in (65, 66):
+        sim = make_sim(s, n, 24, precision, "centroid", steps_per_launch=K, launches_per_poll=4, stats=True,
+                       trace_capacity=0)
+        sim.engine.handle.call("bd_set_launch", group, 128)
+        res = sim.run()
+        outs.append((sim.outcomes(), res.sim_data["min_dist"]))
+        sim.engine.close()
+    for x, y in zip(outs[0][0], outs[1][0]):
+        np.testing.assert_array_equal(x, y)
+    np.testing.assert_array_equal(outs[0][1], outs[1][1])
