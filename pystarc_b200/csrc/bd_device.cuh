@@ -381,9 +381,15 @@ __device__ __forceinline__ StencilOut<FT, CH> stencil(const DevGrid& g, PT x, PT
   const float* d = g.data;
   // centre rows (cx+i, cy+j): three z nodes starting at zb
   const int zb = lz ? cz - 1 : cz;
-  const int zc = lz ? 1 : 0;  // position of node cz inside the three-node run
-  const int ze = lz ? 0 : 2;  // position of the extra z node
-  float r[2][2][3][CH], xe[2][2][CH], ye[2][2][CH];
+  // the nodes: centre cube v, extra x plane xe, extra y row ye, extra z nodes zx (each path fills them
+  // with compile-time indices: an array indexed by lz would live in local memory)
+  float v[2][2][2][CH], xe[2][2][CH], ye[2][2][CH], zx[2][2][CH];
+  // a three-node z run starting at zb: nodes cz, cz + 1 and the extra one
+  auto split_run = [&](int i, int j, int c, float a, float b, float d3) {
+    v[i][j][0][c] = lz ? b : a;
+    v[i][j][1][c] = lz ? d3 : b;
+    zx[i][j][c] = lz ? a : d3;
+  };
   if (CH == 1 && g.cube) {
     // cube copy: the centre block, the x-extra face, the y-extra and z-extra edges in four loads
     // (three with the xy records: the x face and the y edge of this cell half come in one)
@@ -404,9 +410,9 @@ __device__ __forceinline__ StencilOut<FT, CH> stencil(const DevGrid& g, PT x, PT
     for (int i = 0; i < 2; ++i)
 #pragma unroll
       for (int j = 0; j < 2; ++j) {
-        r[i][j][zc][0] = c8[4 * i + 2 * j];
-        r[i][j][zc + 1][0] = c8[4 * i + 2 * j + 1];
-        r[i][j][ze][0] = z8[4 * i + 2 * j];
+        v[i][j][0][0] = c8[4 * i + 2 * j];
+        v[i][j][1][0] = c8[4 * i + 2 * j + 1];
+        zx[i][j][0] = z8[4 * i + 2 * j];
       }
     if (g.xy) {
       float e8[8];
@@ -455,17 +461,11 @@ __device__ __forceinline__ StencilOut<FT, CH> stencil(const DevGrid& g, PT x, PT
         const int n = (cx + i) * syz + (cy + j) * nz + zb;
         const float4 t = __ldg(w + n);
         if constexpr (CH == 1) {
-          r[i][j][0][0] = t.x;
-          r[i][j][1][0] = t.y;
-          r[i][j][2][0] = t.z;
+          split_run(i, j, 0, t.x, t.y, t.z);
         } else {
           const float4 u = __ldg(w + n + 2);
-          r[i][j][0][0] = t.x;
-          r[i][j][0][1] = t.y;
-          r[i][j][1][0] = t.z;
-          r[i][j][1][1] = t.w;
-          r[i][j][2][0] = u.x;
-          r[i][j][2][1] = u.y;
+          split_run(i, j, 0, t.x, t.z, u.x);
+          split_run(i, j, 1, t.y, t.w, u.y);
         }
       }
     float4 tx[2], ty[2];
@@ -497,8 +497,11 @@ __device__ __forceinline__ StencilOut<FT, CH> stencil(const DevGrid& g, PT x, PT
 #pragma unroll
       for (int j = 0; j < 2; ++j) {
         const int base = ((cx + i) * syz + (cy + j) * nz + zb) * CH;
+        float r[3][CH];
 #pragma unroll
-        for (int k = 0; k < 3; ++k) ld<CH>(d + base + k * CH, r[i][j][k]);
+        for (int k = 0; k < 3; ++k) ld<CH>(d + base + k * CH, r[k]);
+#pragma unroll
+        for (int c = 0; c < CH; ++c) split_run(i, j, c, r[0][c], r[1][c], r[2][c]);
       }
     if (CH == 2 && g.ptex) {
       // the eight extra nodes through the texture path, the twelve centre-row nodes above through LSU
@@ -538,47 +541,38 @@ __device__ __forceinline__ StencilOut<FT, CH> stencil(const DevGrid& g, PT x, PT
   StencilOut<FT, CH> o;
 #pragma unroll
   for (int c = 0; c < CH; ++c) {
-    FT v[2][2][2], zx[2][2];
-#pragma unroll
-    for (int i = 0; i < 2; ++i)
-#pragma unroll
-      for (int j = 0; j < 2; ++j) {
-        v[i][j][0] = (FT)r[i][j][zc][c];
-        v[i][j][1] = (FT)r[i][j][zc + 1][c];
-        zx[i][j] = (FT)r[i][j][ze][c];
-      }
     FT phi = 0, Dx = 0, Dy = 0, Dz = 0;
 #pragma unroll
     for (int i = 0; i < 2; ++i)
 #pragma unroll
       for (int j = 0; j < 2; ++j)
 #pragma unroll
-        for (int k = 0; k < 2; ++k) phi += wx[i] * wy[j] * wz[k] * v[i][j][k];
+        for (int k = 0; k < 2; ++k) phi += wx[i] * wy[j] * wz[k] * (FT)v[i][j][k][c];
 #pragma unroll
     for (int j = 0; j < 2; ++j)
 #pragma unroll
       for (int k = 0; k < 2; ++k) {
-        const FT d0 = v[1][j][k] - v[0][j][k];
+        const FT v0 = (FT)v[0][j][k][c], v1 = (FT)v[1][j][k][c], d0 = v1 - v0;
         const FT e = (FT)xe[j][k][c];
-        const FT de = lx ? (v[0][j][k] - e) : (e - v[1][j][k]);
+        const FT de = lx ? (v0 - e) : (e - v1);
         Dx += wy[j] * wz[k] * (((FT)1 - ax) * d0 + ax * de);
       }
 #pragma unroll
     for (int i = 0; i < 2; ++i)
 #pragma unroll
       for (int k = 0; k < 2; ++k) {
-        const FT d0 = v[i][1][k] - v[i][0][k];
+        const FT v0 = (FT)v[i][0][k][c], v1 = (FT)v[i][1][k][c], d0 = v1 - v0;
         const FT e = (FT)ye[i][k][c];
-        const FT de = ly ? (v[i][0][k] - e) : (e - v[i][1][k]);
+        const FT de = ly ? (v0 - e) : (e - v1);
         Dy += wx[i] * wz[k] * (((FT)1 - ay) * d0 + ay * de);
       }
 #pragma unroll
     for (int i = 0; i < 2; ++i)
 #pragma unroll
       for (int j = 0; j < 2; ++j) {
-        const FT d0 = v[i][j][1] - v[i][j][0];
-        const FT e = zx[i][j];
-        const FT de = lz ? (v[i][j][0] - e) : (e - v[i][j][1]);
+        const FT v0 = (FT)v[i][j][0][c], v1 = (FT)v[i][j][1][c], d0 = v1 - v0;
+        const FT e = (FT)zx[i][j][c];
+        const FT de = lz ? (v0 - e) : (e - v1);
         Dz += wx[i] * wy[j] * (((FT)1 - az) * d0 + az * de);
       }
     o.phi[c] = phi;
