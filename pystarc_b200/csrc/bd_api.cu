@@ -659,21 +659,12 @@ const KernelTable& table_for(int prec, int torque) {
   return tables[(prec == BD_PREC_FP64 ? 0 : 2) + (torque == BD_TORQUE_CENTROID ? 1 : 0)];
 }
 
-// which: 0 evaluation of poses, 1 evaluation with explicit atoms, 2 stepper
-void* kernel_for(int prec, int G, int torque, int which) {
+void* stepper_for(int prec, int G, int torque) {
   const KernelTable& t = table_for(prec, torque);
-  if (G == BD_GROUP_SPLIT) {
-    // the stepper has kernels of its own; the parity kernels use a full-warp group
-    if (which == 2) return t.split.mid;
-    G = 32;
-  }
-  if (G == BD_GROUP_WARP || G == BD_GROUP_WARP_CAPPED) {
-    // warp-cooperative stepper; the parity kernels use a full-warp group (same sweep code)
-    if (which == 2) return G == BD_GROUP_WARP ? t.warp : t.warp_capped;
-    G = 32;
-  }
+  if (G == BD_GROUP_SPLIT) return t.split.mid;
+  if (G == BD_GROUP_WARP || G == BD_GROUP_WARP_CAPPED) return G == BD_GROUP_WARP ? t.warp : t.warp_capped;
   for (int i = 0; i < 5; ++i)
-    if (kGroups[i] == G) return which == 0 ? t.pose[i] : which == 1 ? t.atoms[i] : t.step[i];
+    if (kGroups[i] == G) return t.step[i];
   return nullptr;
 }
 
@@ -753,14 +744,6 @@ int launch_group_for(const BdHandle* h, int overlap) {
 
 int launch_group(const BdHandle* h) { return launch_group_for(h, h->sp.overlap); }
 
-int eval_grid_blocks(BdHandle* h, long long n, int G, int block) {
-  const long long groups = (n + 0);
-  const long long per_block = block / G;
-  long long blocks = (groups + per_block - 1) / per_block;
-  blocks = std::min<long long>(blocks, (long long)h->n_sm * 64);
-  return (int)std::max<long long>(blocks, 1);
-}
-
 int persistent_blocks(BdHandle* h, void* fn, int block, size_t smem = 0) {
   int per_sm = 0;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, block, smem) != cudaSuccess || per_sm < 1) per_sm = 1;
@@ -792,6 +775,40 @@ size_t stepper_smem(const DevSystem& S, const DevSim& P, void* fn) {
   if (fn && cudaFuncGetAttributes(&a, fn) == cudaSuccess && (int)b > a.maxDynamicSharedSizeBytes)
     cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)b);
   return b;
+}
+
+// Forces of a batch of poses.  Groups of 1 to 16 lanes (tiny ligands with nothing to sweep, or the
+// caller's choice) run one kernel; whole warps run the split force code.  A block per pose is the faster
+// up to 24 poses per SM (a warp per pose takes 50-90 us however few there are): protein + small ligand
+// FP64, 37 poses 53 us before -> 21, 592 55 -> 30, 1,500 68 -> 58 (100 with a warp per pose); 3,000 poses
+// by warps 124 -> 135, 20,000 607 -> 389, 100,000 mixed 1,240 -> 920; protein-protein FP64 37 poses
+// 168 -> 42, 6,000 1,119 -> 808.
+int eval_batch(BdHandle* h, PoseBatch P, int prec, int torque, cudaStream_t s) {
+  const KernelTable& t = table_for(prec, torque);
+  const int G = launch_group(h);
+  for (int i = 0; i < 4; ++i)
+    if (kGroups[i] == G) {
+      const int block = 128;
+      const long long per_block = block / G;
+      const int blocks = (int)std::min<long long>((P.n + per_block - 1) / per_block, (long long)h->n_sm * 64);
+      unsigned long long* ctr = nullptr;
+      void* pose_args[] = {&h->S, &P.n, &P.cen, &P.rot, &P.rot_is_matrix, &P.F, &P.T, &P.E, &ctr};
+      void* atom_args[] = {&h->S, &P.n, &P.atoms, &P.rot, &P.cen, &P.F, &P.T, &P.E};
+      CK(h, cudaLaunchKernel(P.atoms ? t.atoms[i] : t.pose[i], dim3(blocks), dim3(block),
+                             P.atoms ? atom_args : pose_args, 0, s));
+      return BD_OK;
+    }
+  void* args[] = {&h->S, &P};
+  if (P.n <= (long long)kBlockPoses * h->n_sm && !h->S.wca) {
+    CK(h, cudaLaunchKernel(t.pose_block, dim3((unsigned)P.n), dim3(256), args, 0, s));
+    return BD_OK;
+  }
+  const long long want = (P.n + 7) / 8;  // a warp per pose
+  const int b_fwd = (int)std::min<long long>(want, persistent_blocks(h, t.pose_fwd, 256)),
+            b_rev = (int)std::min<long long>(want, persistent_blocks(h, t.pose_rev, 256));
+  CK(h, cudaLaunchKernel(t.pose_fwd, dim3(b_fwd), dim3(256), args, 0, s));
+  if (h->S.born_rev && (h->S.terms & BD_TERM_REV_BORN)) CK(h, cudaLaunchKernel(t.pose_rev, dim3(b_rev), dim3(256), args, 0, s));
+  return BD_OK;
 }
 
 }  // namespace
@@ -942,15 +959,7 @@ int bd_eval_forces(BdHandle* h, int64_t n, const double* cen, const double* rot,
   int rc = finalize(h);
   if (rc) return rc;
   if (n == 0) return BD_OK;
-  const int G = launch_group(h);
-  const int block = 128;
-  void* fn = kernel_for(prec, G, torque, 0);
-  unsigned long long* ctr = nullptr;
-  long long nn = n;
-  int rim = rot_is_matrix;
-  void* args[] = {&h->S, &nn, &cen, &rot, &rim, &F, &T, &E, &ctr};
-  CK(h, cudaLaunchKernel(fn, dim3(eval_grid_blocks(h, n, G, block)), dim3(block), args, 0, pick(h, stream)));
-  return BD_OK;
+  return eval_batch(h, PoseBatch{n, cen, rot, rot_is_matrix, nullptr, F, T, E}, prec, torque, pick(h, stream));
 }
 
 int bd_eval_forces_atoms(BdHandle* h, int64_t n, const double* pos, const double* R, const double* cen, double* F,
@@ -964,13 +973,7 @@ int bd_eval_forces_atoms(BdHandle* h, int64_t n, const double* pos, const double
   int rc = finalize(h);
   if (rc) return rc;
   if (n == 0) return BD_OK;
-  const int G = launch_group(h);
-  const int block = 128;
-  void* fn = kernel_for(prec, G, torque, 1);
-  long long nn = n;
-  void* args[] = {&h->S, &nn, &pos, &R, &cen, &F, &T, &E};
-  CK(h, cudaLaunchKernel(fn, dim3(eval_grid_blocks(h, n, G, block)), dim3(block), args, 0, pick(h, stream)));
-  return BD_OK;
+  return eval_batch(h, PoseBatch{n, cen, R, 1, pos, F, T, E}, prec, torque, pick(h, stream));
 }
 
 int bd_eval_overlap(BdHandle* h, int64_t n, const double* cen, int8_t* out, void* stream) {
@@ -1119,7 +1122,7 @@ int bd_get_launch(BdHandle* h, int* group, int* block, int* grid) {
   if (group) *group = G;
   if (block) *block = h->block;
   if (grid) {
-    void* fn = kernel_for(h->sp.precision, G, h->sp.torque_mode, 2);
+    void* fn = stepper_for(h->sp.precision, G, h->sp.torque_mode);
     *grid = fn ? resident_blocks(h, G, fn, stepper_smem(h->S, h->P, fn)) : 0;
   }
   return BD_OK;
@@ -1158,7 +1161,7 @@ int bd_sim_configure(BdHandle* h, const BdSimParams* p) {
   h->sp = *p;
   // live-slot capacity
   const int G = launch_group(h);
-  void* fn = kernel_for(p->precision, G, p->torque_mode, 2);
+  void* fn = stepper_for(p->precision, G, p->torque_mode);
   DevSim probe{};
   probe.stats = p->stats;
   const long long resident =
@@ -1505,7 +1508,7 @@ int build_graphs(BdHandle* h, int K) {
       cudaGraphExecDestroy(g);
       g = nullptr;
     }
-  void* fn = kernel_for(h->sp.precision, G, h->sp.torque_mode, 2);
+  void* fn = stepper_for(h->sp.precision, G, h->sp.torque_mode);
   const size_t smem = stepper_smem(h->S, h->P, fn);
   const int blocks = resident_blocks(h, G, fn, smem);
   const int sblocks = h->sur ? surrogate_blocks(h) : 0;
@@ -1846,7 +1849,7 @@ int bd_internal_run_noalloc(BdHandle* h, const BdSimParams* p, unsigned char* sc
   CK(h, cudaStreamSynchronize(s));
   int G = launch_group_for(h, p->overlap);
   if (G == BD_GROUP_SPLIT) G = BD_GROUP_WARP_CAPPED;  // the split stepper's scratch would need allocating
-  void* fn = kernel_for(p->precision, G, p->torque_mode, 2);
+  void* fn = stepper_for(p->precision, G, p->torque_mode);
   const size_t smem = stepper_smem(h->S, P, fn);
   const int blocks = persistent_blocks(h, fn, h->block, smem);
   int cur = 0;

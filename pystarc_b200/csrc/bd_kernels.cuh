@@ -328,10 +328,17 @@ __device__ void group_contact(const DevSystem& S, const double c[3], int lane, u
   }
 }
 
+// CALL: the far-field as a function call, for kernels outside whose loops the compiler would otherwise
+// fuse its products and sums differently and round the last bit another way.
+template <typename FT>
+__device__ __noinline__ void farfield_call(const DevSystem& S, double x, double y, double z, FT q, FT f[3], FT& e) {
+  farfield<FT>(S, x, y, z, q, f, e);
+}
+
 // Force (and energy) on one charged ligand atom at lab position x: the finest electrostatic grid that
 // holds it or the far-field, and Born direction 1 (gpu_batch_engine.py:556-582).  False if the atom's
 // terms are switched off.
-template <typename FT, bool ENERGY>
+template <typename FT, bool ENERGY, bool CALL = false>
 __device__ __forceinline__ bool ligand_atom(const DevSystem& S, double charge, const double x[3], bool t_grid,
                                             bool t_ff, FT fa[3], FT& ea, unsigned& ng, unsigned& nf) {
   const FT q = (FT)charge;
@@ -365,7 +372,8 @@ __device__ __forceinline__ bool ligand_atom(const DevSystem& S, double charge, c
       }
     } else if (S.has_yukawa && t_ff) {
       FT ff[3], ef;
-      farfield<FT>(S, x[0], x[1], x[2], q, ff, ef);
+      if constexpr (CALL) farfield_call<FT>(S, x[0], x[1], x[2], q, ff, ef);
+      else farfield<FT>(S, x[0], x[1], x[2], q, ff, ef);
       fa0 = ff[0];
       fa1 = ff[1];
       fa2 = ff[2];

@@ -335,7 +335,7 @@ __device__ __forceinline__ void group_forward(const DevSystem& S, const PosFn& p
       double ro[3], x[3];
       pos(i, a, ro, x);
       FT fa[3], ea;
-      if (fabs(a.w) >= 1e-9 && ligand_atom<FT, ENERGY>(S, a.w, x, t_grid, t_ff, fa, ea, cnt.grid, cnt.ff)) {
+      if (fabs(a.w) >= 1e-9 && ligand_atom<FT, ENERGY, ENERGY>(S, a.w, x, t_grid, t_ff, fa, ea, cnt.grid, cnt.ff)) {
 #pragma unroll
         for (int d = 0; d < 3; ++d) f[d] = (double)fa[d];
         if (ENERGY) e = (double)ea;
@@ -365,6 +365,7 @@ __device__ __forceinline__ void group_forward(const DevSystem& S, const PosFn& p
 #pragma unroll
   for (int k = 0; k < 4; ++k)
     if (gw + k * W < NC) tot[k] = gsum<32>(tot[k], 0xffffffffu);
+  group_sync(bar, 32 * W);  // every row is read before the next pose writes one
 }
 
 // Warps per pose of the forward forces of a large ligand, for a list of n poses on n_warps warps: only
