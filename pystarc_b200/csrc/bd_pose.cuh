@@ -155,7 +155,7 @@ __global__ void __launch_bounds__(256, sizeof(FT) == 4 ? 4 : 2) pose_rev_kernel(
     if (!needs_reverse(S, c)) continue;
     const BatchSrc src{P, t};
     double r[3] = {0, 0, 0}, u[3] = {0, 0, 0};
-    lean_reverse_born<FT, TORQUE>(S, src, lane, bufs[warp], r, u, nr);
+    lean_reverse_born<FT, TORQUE, true>(S, src, lane, bufs[warp], r, u, nr);
 #pragma unroll
     for (int i = 0; i < 3; ++i) {
       r[i] = gsum<32>(r[i], FULL);

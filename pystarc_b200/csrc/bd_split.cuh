@@ -489,13 +489,15 @@ struct RevPose {
   }
 
   // Receptor atom idx is charged and inside the box; e = its ligand-frame position and charge.
+  static __device__ __forceinline__ V4 atom(const DevSystem& S, int idx) {
+    if constexpr (sizeof(FT) == 4) return S.rec_f[idx];
+    else return S.rec[idx];
+  }
+
   template <class SRC>
-  __device__ __forceinline__ bool candidate(const DevSystem& S, const SRC& src, int idx, V4& e) const {
+  __device__ __forceinline__ bool candidate(const DevSystem& S, const SRC& src, int idx, const V4& at, V4& e) const {
     const DevGrid& g = S.lig_born;
     const FT lox = (FT)g.lox, loy = (FT)g.loy, loz = (FT)g.loz, hix = (FT)g.hix, hiy = (FT)g.hiy, hiz = (FT)g.hiz;
-    V4 at;
-    if constexpr (sizeof(FT) == 4) at = S.rec_f[idx];
-    else at = S.rec[idx];
     if (!(fabs(at.w) >= (FT)1e-9)) return false;
     const FT d0 = (FT)at.x - cx, d1 = (FT)at.y - cy, d2 = (FT)at.z - cz;
     const FT l0 = Rt[0] * d0 + Rt[3] * d1 + Rt[6] * d2;
@@ -523,7 +525,11 @@ struct RevPose {
 // receptor chunks culled against the ligand Born grid's margin box in the ligand frame, in-box
 // atoms gathered into `buf` and drained 32 at a time.  Adds this lane's share of the sums to
 // r (ligand frame) and u; the caller reduces over the warp.
-template <typename FT, bool TORQUE, class SRC>
+// AHEAD: the next hit chunk's atoms load while one chunk's are tested.  In FP64 and in the evaluation
+// kernel that pays (30,011 FP64 trajectories 117 -> 113 ms of GPU time, 20,000 FP64 poses 390 -> 351 us,
+// mixed 267 -> 248); in the mixed stepper the registers it takes from the 64 cost as much as it gains
+// (150,000 trajectories 327 -> 332 ms).
+template <typename FT, bool TORQUE, bool AHEAD, class SRC>
 __device__ __forceinline__ void lean_reverse_born(const DevSystem& S, const SRC& src, int lane,
                                                   typename Vec4<FT>::type* buf, double r[3], double u[3],
                                                   unsigned& nr) {
@@ -533,27 +539,41 @@ __device__ __forceinline__ void lean_reverse_born(const DevSystem& S, const SRC&
   const RevPose<FT> pose(src);
   FT rs0 = 0, rs1 = 0, rs2 = 0;
   int k0 = 0, head = 0;
+  int kk = -1;  // the chunk whose atoms `at` holds, -1: none
   unsigned hits = 0;
+  V4 at{};
   bool done = false;
   for (;;) {
     // gather until the buffer has no room for another chunk, or every chunk is done
     while (head <= kSplitBuf<FT> - 32) {
-      if (!hits) {
-        if (k0 >= S.n_chunks) {
-          done = true;
-          break;
+      if (kk < 0) {
+        if (!hits) {
+          if (k0 >= S.n_chunks) {
+            done = true;
+            break;
+          }
+          hits = __ballot_sync(FULL, pose.hits(S, k0 + lane));
+          k0 += 32;
+          continue;
         }
-        hits = __ballot_sync(FULL, pose.hits(S, k0 + lane));
-        k0 += 32;
-        continue;
+        kk = k0 - 32 + __ffs(hits) - 1;
+        hits &= hits - 1;
+        at = pose.atom(S, kk * BD_CHUNK + lane);
       }
-      const int kk = k0 - 32 + __ffs(hits) - 1;
-      hits &= hits - 1;
+      int kn = -1;
+      V4 an = at;
+      if (AHEAD) {
+        kn = hits ? k0 - 32 + __ffs(hits) - 1 : -1;
+        hits &= hits - 1;
+        if (kn >= 0) an = pose.atom(S, kn * BD_CHUNK + lane);
+      }
       V4 ent{};
-      const bool cand = pose.candidate(S, src, kk * BD_CHUNK + lane, ent);
+      const bool cand = pose.candidate(S, src, kk * BD_CHUNK + lane, at, ent);
       const unsigned m = __ballot_sync(FULL, cand);
       if (cand) buf[head + __popc(m & ((1u << lane) - 1u))] = ent;
       head += __popc(m);
+      at = an;
+      kk = kn;
     }
     __syncwarp();
     // drain whole groups of 32 (everything once the chunks are done): entry e by lane e mod 32
@@ -681,7 +701,8 @@ __device__ __forceinline__ void group_reverse_born(const DevSystem& S, const SRC
         const int nth = h - __shfl_sync(FULL, before, ml);
         const unsigned at =
             __ballot_sync(FULL, ((m >> lane) & 1u) && __popc(m & ((1u << lane) - 1u)) == nth);
-        cand = pose.candidate(S, src, (c0 + 32 * ml + __ffs(at) - 1) * BD_CHUNK + lane, ent);
+        const int idx = (c0 + 32 * ml + __ffs(at) - 1) * BD_CHUNK + lane;
+        cand = pose.candidate(S, src, idx, pose.atom(S, idx), ent);
       }
       const unsigned m = __ballot_sync(FULL, cand);
       if (lane == 0) cnt[flip * 8 + gw] = __popc(m);
@@ -744,7 +765,7 @@ __global__ void __launch_bounds__(256, sizeof(FT) == 4 ? 4 : 2) split_rev_kernel
     const DevSystem& S = T.sys(T.locate(id));
     double r[3] = {0, 0, 0}, u[3] = {0, 0, 0};
     if (W == 1) {
-      lean_reverse_born<FT, TORQUE>(S, SlotSrc{B, slot}, lane, bufs[warp], r, u, nr);
+      lean_reverse_born<FT, TORQUE, sizeof(FT) == 8>(S, SlotSrc{B, slot}, lane, bufs[warp], r, u, nr);
     } else {
       V4* buf = bufs[grp * W];
       group_reverse_born<FT, TORQUE>(S, SlotSrc{B, slot}, lane, gw, W, 1 + grp, buf, TORQUE ? vals[grp * W] : buf,
