@@ -205,6 +205,12 @@ void grid_to_dev(const GridHost& g, const float* dptr, int ch, DevGrid& d) {
   d.isxf = (float)d.isx;
   d.isyf = (float)d.isy;
   d.iszf = (float)d.isz;
+  d.loxf = (float)d.lox;
+  d.loyf = (float)d.loy;
+  d.lozf = (float)d.loz;
+  d.hixf = (float)d.hix;
+  d.hiyf = (float)d.hiy;
+  d.hizf = (float)d.hiz;
 }
 
 int upload_floats(BdHandle* h, const float* src, size_t n, const float** out) {
@@ -468,6 +474,12 @@ int finalize(BdHandle* h) {
     for (int i = 0; i < 9; ++i) S.quad[i] = fp.quadrupole[i];
     S.inv_fpe = 1.0 / fp.four_pi_eps;
   }
+  S.V_factor_f = (float)S.V_factor;
+  S.inv_debye_f = (float)S.inv_debye;
+  S.inv_fpe_f = (float)S.inv_fpe;
+  S.alpha_f = (float)S.alpha;
+  for (int i = 0; i < 3; ++i) S.dip_f[i] = (float)S.dip[i];
+  for (int i = 0; i < 9; ++i) S.quad_f[i] = (float)S.quad[i];
   // grids: finest first (stable on the x spacing), reference dropping rules
   std::vector<const GridHost*> el, bo, lb;
   for (const GridHost& g : h->grids[BD_GRID_ELEC]) el.push_back(&g);

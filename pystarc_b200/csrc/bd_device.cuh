@@ -60,8 +60,18 @@ struct DevGrid {
   double ox, oy, oz;
   double isx, isy, isz;  // 1/spacing
   double lox, loy, loz, hix, hiy, hiz;  // strict margin box
-  float oxf, oyf, ozf, isxf, isyf, iszf;  // FP32 origin and 1/spacing (the FP32-position stencil)
+  // FP32 copies, rounded once on the host: converting a double takes the slow conversion pipe for
+  // every stencil and every box test (FP32 arithmetic reads these, by `in`)
+  float oxf, oyf, ozf, isxf, isyf, iszf;
+  float loxf, loyf, lozf, hixf, hiyf, hizf;
 };
+
+// A constant in the arithmetic's type: the double, or its FP32 copy.
+template <typename FT>
+__device__ __forceinline__ FT in(double d, float f) {
+  if constexpr (sizeof(FT) == 4) return f;
+  else return d;
+}
 
 struct DevSystem {
   // ligand (body frame = about the ligand centroid)
@@ -98,6 +108,7 @@ struct DevSystem {
   double V_factor, inv_debye, inv_fpe;
   double dip[3], quad[9];
   double alpha;
+  float V_factor_f, inv_debye_f, inv_fpe_f, dip_f[3], quad_f[9], alpha_f;  // FP32 copies
   // WCA contact term (wca = 0: off): epsilon, centroid activation radius, largest pair cutoff
   int wca;
   double wca_eps, wca_act, wca_cut;
@@ -576,9 +587,9 @@ __device__ __forceinline__ StencilOut<FT, CH> stencil(const DevGrid& g, PT x, PT
         Dz += wx[i] * wy[j] * (((FT)1 - az) * d0 + az * de);
       }
     o.phi[c] = phi;
-    o.gx[c] = Dx * (FT)g.isx;
-    o.gy[c] = Dy * (FT)g.isy;
-    o.gz[c] = Dz * (FT)g.isz;
+    o.gx[c] = Dx * in<FT>(g.isx, g.isxf);
+    o.gy[c] = Dy * in<FT>(g.isy, g.isyf);
+    o.gz[c] = Dz * in<FT>(g.isz, g.iszf);
   }
   return o;
 }
@@ -594,24 +605,24 @@ __device__ __forceinline__ void farfield(const DevSystem& S, double xd, double y
   const FT r = sqrt(x * x + y * y + z * z);
   const FT sr = r > (FT)1 ? r : (FT)1;
   const FT inv = (FT)1 / sr;
-  const FT il = (FT)S.inv_debye;
+  const FT il = in<FT>(S.inv_debye, S.inv_debye_f);
   const FT ex = exp(-sr * il);
   const FT rx = x * inv, ry = y * inv, rz = z * inv;
-  const FT Vf = (FT)S.V_factor;
+  const FT Vf = in<FT>(S.V_factor, S.V_factor_f);
   FT phi = Vf * ex * inv;
   FT dphi = Vf * ex * (-inv * inv - inv * il);
   if (S.use_dip) {
-    const FT pr = rx * (FT)S.dip[0] + ry * (FT)S.dip[1] + rz * (FT)S.dip[2];
-    const FT ifpe = (FT)S.inv_fpe;
+    const FT pr = rx * in<FT>(S.dip[0], S.dip_f[0]) + ry * in<FT>(S.dip[1], S.dip_f[1]) + rz * in<FT>(S.dip[2], S.dip_f[2]);
+    const FT ifpe = in<FT>(S.inv_fpe, S.inv_fpe_f);
     phi += pr * ifpe * inv * inv * ((FT)1 + sr * il) * ex;
     dphi += pr * ifpe * ex * ((FT)-2 * inv * inv * inv - (FT)2 * inv * inv * il - inv * il * il);
   }
   if (S.use_quad) {
-    const FT qx = (FT)S.quad[0] * rx + (FT)S.quad[1] * ry + (FT)S.quad[2] * rz;
-    const FT qy = (FT)S.quad[3] * rx + (FT)S.quad[4] * ry + (FT)S.quad[5] * rz;
-    const FT qz = (FT)S.quad[6] * rx + (FT)S.quad[7] * ry + (FT)S.quad[8] * rz;
+    const FT qx = in<FT>(S.quad[0], S.quad_f[0]) * rx + in<FT>(S.quad[1], S.quad_f[1]) * ry + in<FT>(S.quad[2], S.quad_f[2]) * rz;
+    const FT qy = in<FT>(S.quad[3], S.quad_f[3]) * rx + in<FT>(S.quad[4], S.quad_f[4]) * ry + in<FT>(S.quad[5], S.quad_f[5]) * rz;
+    const FT qz = in<FT>(S.quad[6], S.quad_f[6]) * rx + in<FT>(S.quad[7], S.quad_f[7]) * ry + in<FT>(S.quad[8], S.quad_f[8]) * rz;
     const FT rQr = rx * qx + ry * qy + rz * qz;
-    const FT ifpe = (FT)S.inv_fpe;
+    const FT ifpe = in<FT>(S.inv_fpe, S.inv_fpe_f);
     const FT i2 = inv * inv, i3 = i2 * inv;
     phi += rQr * ifpe * i3 * ((FT)1 + sr * il + sr * sr * il * il * ((FT)1 / (FT)3)) * ex;
     dphi += rQr * ifpe * ex *

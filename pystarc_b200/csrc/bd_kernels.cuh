@@ -136,9 +136,10 @@ __device__ __forceinline__ void warp_reverse_born(const DevSystem& S, const doub
   V4* ring = rings[threadIdx.x >> 5];
   const unsigned FULL = 0xffffffffu;
   const DevGrid& g = S.lig_born;
-  const FT alpha = (FT)S.alpha;
+  const FT alpha = in<FT>(S.alpha, S.alpha_f);
   const FT Rt[9] = {(FT)R[0], (FT)R[1], (FT)R[2], (FT)R[3], (FT)R[4], (FT)R[5], (FT)R[6], (FT)R[7], (FT)R[8]};
-  const FT lox = (FT)g.lox, loy = (FT)g.loy, loz = (FT)g.loz, hix = (FT)g.hix, hiy = (FT)g.hiy, hiz = (FT)g.hiz;
+  const FT lox = in<FT>(g.lox, g.loxf), loy = in<FT>(g.loy, g.loyf), loz = in<FT>(g.loz, g.lozf);
+  const FT hix = in<FT>(g.hix, g.hixf), hiy = in<FT>(g.hiy, g.hiyf), hiz = in<FT>(g.hiz, g.hizf);
   unsigned head = 0, tail = 0;  // warp-uniform ring cursors
   FT rs0 = 0, rs1 = 0, rs2 = 0;  // per-lane sums in FT (at most a few dozen terms per lane)
   auto drain = [&](unsigned count) {
@@ -350,8 +351,9 @@ __device__ __forceinline__ bool ligand_atom(const DevSystem& S, double charge, c
       gi = k;
       break;
     }
-  const bool bin = S.has_born && in_box(S.born, x[0], x[1], x[2]);
-  const FT cb = (FT)S.alpha * q * q;
+  // a paired Born grid has the finest electrostatic grid's box
+  const bool bin = S.paired ? gi == 0 : S.has_born && in_box(S.born, x[0], x[1], x[2]);
+  const FT cb = in<FT>(S.alpha, S.alpha_f) * q * q;
   if (gi == 0 && bin && S.paired) {
     if (!t_grid) return false;
     const StencilOut<FT, 2> s = stencil<FT, 2>(S.pair, x[0], x[1], x[2]);
@@ -483,7 +485,7 @@ __device__ void group_forces(const DevSystem& S, const double c[3], const double
           if (!in_box(S.lig_born, l0, l1, l2)) continue;
           const StencilOut<FT, 1> s = stencil<FT, 1>(S.lig_born, l0, l1, l2);
           const FT qr = (FT)at.w;
-          const FT cf = -(FT)S.alpha * qr * qr;
+          const FT cf = -in<FT>(S.alpha, S.alpha_f) * qr * qr;
           const FT g0 = cf * s.gx[0], g1 = cf * s.gy[0], g2 = cf * s.gz[0];
           r0 += (double)g0;
           r1 += (double)g1;

@@ -472,7 +472,8 @@ struct RevPose {
   __device__ __forceinline__ bool hits(const DevSystem& S, int k) const {
     if (k >= S.n_chunks) return false;
     const DevGrid& g = S.lig_born;
-    const FT lox = (FT)g.lox, loy = (FT)g.loy, loz = (FT)g.loz, hix = (FT)g.hix, hiy = (FT)g.hiy, hiz = (FT)g.hiz;
+    const FT lox = in<FT>(g.lox, g.loxf), loy = in<FT>(g.loy, g.loyf), loz = in<FT>(g.loz, g.lozf);
+    const FT hix = in<FT>(g.hix, g.hixf), hiy = in<FT>(g.hiy, g.hiyf), hiz = in<FT>(g.hiz, g.hizf);
     V4 sp;
     if constexpr (sizeof(FT) == 4) sp = S.chunks_f[k];
     else sp = S.chunks[k];
@@ -497,7 +498,8 @@ struct RevPose {
   template <class SRC>
   __device__ __forceinline__ bool candidate(const DevSystem& S, const SRC& src, int idx, const V4& at, V4& e) const {
     const DevGrid& g = S.lig_born;
-    const FT lox = (FT)g.lox, loy = (FT)g.loy, loz = (FT)g.loz, hix = (FT)g.hix, hiy = (FT)g.hiy, hiz = (FT)g.hiz;
+    const FT lox = in<FT>(g.lox, g.loxf), loy = in<FT>(g.loy, g.loyf), loz = in<FT>(g.loz, g.lozf);
+    const FT hix = in<FT>(g.hix, g.hixf), hiy = in<FT>(g.hiy, g.hiyf), hiz = in<FT>(g.hiz, g.hizf);
     if (!(fabs(at.w) >= (FT)1e-9)) return false;
     const FT d0 = (FT)at.x - cx, d1 = (FT)at.y - cy, d2 = (FT)at.z - cz;
     const FT l0 = Rt[0] * d0 + Rt[3] * d1 + Rt[6] * d2;
@@ -578,7 +580,7 @@ __device__ __forceinline__ void lean_reverse_born(const DevSystem& S, const SRC&
     __syncwarp();
     // drain whole groups of 32 (everything once the chunks are done): entry e by lane e mod 32
     const int n_drain = done ? head : (head & ~31);
-    const FT alpha = (FT)S.alpha;
+    const FT alpha = in<FT>(S.alpha, S.alpha_f);
 #pragma unroll 1
     for (int e = lane; e < n_drain; e += 32) {
       const V4 v = buf[e];
@@ -629,7 +631,7 @@ __device__ __forceinline__ void group_reverse_born(const DevSystem& S, const SRC
   const unsigned FULL = 0xffffffffu;
   const DevGrid& g = S.lig_born;
   const RevPose<FT> pose(src);
-  const FT alpha = (FT)S.alpha;
+  const FT alpha = in<FT>(S.alpha, S.alpha_f);
   FT rs0 = 0, rs1 = 0, rs2 = 0;
   int head = 0, flip = 0;
   // evaluate and sum the first n entries (a multiple of 32, or all of them)
