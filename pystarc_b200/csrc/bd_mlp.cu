@@ -287,30 +287,39 @@ __global__ void loss_finish_kernel(const float* __restrict__ partial, int nb, fl
   }
 }
 
-// Weight gradient of one layer from split partials (summed in split order) and
-// bias gradient as the row sums of dZ^T [out_pad][ldt] over the first n columns.
-__global__ void grad_reduce_kernel(const float* __restrict__ part, int splits, long long split_stride, int ldp,
-                                   int out_real, int in_real, float* __restrict__ gW) {
-  const int total = out_real * in_real;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
-    const int o = i / in_real, c = i % in_real;
-    float s = 0.f;
-    for (int z = 0; z < splits; ++z) s += part[z * split_stride + (size_t)o * ldp + c];
-    gW[i] = s;
-  }
-}
+// Gradients of a layer (blockIdx.y) from its split partials and dZ^T.  Blocks below out_real: the bias
+// gradient of output row o = blockIdx.x, the sum of dZ^T[o][0..n) (n a multiple of 8): thread t adds the
+// 8-element vectors t, t + 256, ... in order, then a fixed-order butterfly per warp and the eight warp
+// sums in order.  The blocks after them: the weight gradient, the partials summed in split order.
+struct GradLayer {
+  const float* part;
+  long long split_stride;
+  int splits, ldp, out_real, in_real;
+  const bf16* dZt;
+  float *gW, *gb;
+};
+struct GradBatch {
+  GradLayer l[kMaxLayers];
+  int n;
+};
 
-// Bias gradient: one 256-thread block per output row o sums dZ^T[o][0..n) (n and ldt
-// multiples of 8): thread t adds the 8-element vectors t, t + 256, ... in order, then a
-// fixed-order butterfly per warp and the eight warp sums in order.
-__global__ void __launch_bounds__(256) bias_grad_kernel(const bf16* __restrict__ dZt, int ldt, int n, int out_real,
-                                                        float* __restrict__ gb) {
+__global__ void __launch_bounds__(256) grad_finish_kernel(const __grid_constant__ GradBatch b) {
   __shared__ float ws[8];
-  const int o = blockIdx.x, tid = threadIdx.x, lane = tid & 31;
-  if (o >= out_real) return;
-  const uint4* row = reinterpret_cast<const uint4*>(dZt + (size_t)o * ldt);
+  const GradLayer& g = b.l[blockIdx.y];
+  const int tid = threadIdx.x, lane = tid & 31;
+  if ((int)blockIdx.x >= g.out_real) {
+    const int total = g.out_real * g.in_real, stride = ((int)gridDim.x - g.out_real) * 256;
+    for (int i = ((int)blockIdx.x - g.out_real) * 256 + tid; i < total; i += stride) {
+      const int o = i / g.in_real, c = i % g.in_real;
+      float s = 0.f;
+      for (int z = 0; z < g.splits; ++z) s += g.part[z * g.split_stride + (size_t)o * g.ldp + c];
+      g.gW[i] = s;
+    }
+    return;
+  }
+  const uint4* row = reinterpret_cast<const uint4*>(g.dZt + (size_t)blockIdx.x * b.n);
   float s = 0.f;
-  for (int v = tid; v < n / 8; v += 256) {
+  for (int v = tid; v < b.n / 8; v += 256) {
     const uint4 u = __ldg(row + v);
     const uint32_t w[4] = {u.x, u.y, u.z, u.w};
 #pragma unroll
@@ -327,7 +336,7 @@ __global__ void __launch_bounds__(256) bias_grad_kernel(const bf16* __restrict__
     float t = 0.f;
 #pragma unroll
     for (int k = 0; k < 8; ++k) t += ws[k];
-    gb[o] = t;
+    g.gb[blockIdx.x] = t;
   }
 }
 
@@ -579,7 +588,7 @@ __host__ __device__ constexpr int gt_stage_bytes(int BN) { return kGtBytesA + BN
 __host__ __device__ constexpr int gt_smem_bytes(int BN) { return kGtStages * gt_stage_bytes(BN) + 8 * kGtStages + 16; }
 
 template <int EPI>
-__global__ void __launch_bounds__(kGtThreads, 1) gemm_nt_tc(GemmArgs g, int BN) {
+__device__ __forceinline__ void gemm_tc_tile(const GemmArgs& g, int BN, int z) {
   extern __shared__ __align__(1024) unsigned char gt_smem[];
   // stage st: A tile at st * stage bytes, B tile right after it
   const int sb = gt_stage_bytes(BN);
@@ -590,8 +599,8 @@ __global__ void __launch_bounds__(kGtThreads, 1) gemm_nt_tc(GemmArgs g, int BN) 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int n0 = blockIdx.x * BN;
   const int M = g.m_dev ? min(g.M, *g.m_dev) : g.M;
-  const int kb = blockIdx.z * g.k_per_split, ke = min(g.K, kb + g.k_per_split);
-  if (blockIdx.y * 128 >= M || kb >= ke) return;  // whole block, before any allocation
+  const int kb = z * g.k_per_split, ke = min(g.K, kb + g.k_per_split);
+  if (n0 >= g.N || blockIdx.y * 128 >= M || kb >= ke) return;  // whole block, before any allocation
   const int nb = min(BN, g.N - n0);  // columns of this block (a multiple of 16)
   const uint32_t ncols = nb <= 32 ? 32 : nb <= 64 ? 64 : nb <= 128 ? 128 : 256;
   if (warp == 0) {
@@ -697,7 +706,7 @@ __global__ void __launch_bounds__(kGtThreads, 1) gemm_nt_tc(GemmArgs g, int BN) 
       for (int e = 0; e < 32; ++e) f[e] = ok ? __uint_as_float(v[e]) : __int_as_float(0x7fc00000);
       if (!valid && !(EPI == EPI_HIDDEN_FWD || EPI == EPI_HIDDEN_BWD)) continue;
       if constexpr (EPI == EPI_PARTIAL) {
-        float* p = g.C + blockIdx.z * g.split_stride + (size_t)r * g.ldc + cb;
+        float* p = g.C + z * g.split_stride + (size_t)r * g.ldc + cb;
 #pragma unroll
         for (int e = 0; e < 32; e += 4)
           if (e < cw) *reinterpret_cast<float4*>(p + e) = make_float4(f[e], f[e + 1], f[e + 2], f[e + 3]);
@@ -762,6 +771,22 @@ __global__ void __launch_bounds__(kGtThreads, 1) gemm_nt_tc(GemmArgs g, int BN) 
     __syncthreads();  // every lane is read before the next tile's MMAs overwrite the accumulator
   }
   if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(ncols));
+}
+
+template <int EPI>
+__global__ void __launch_bounds__(kGtThreads, 1) gemm_nt_tc(GemmArgs g, int BN) {
+  gemm_tc_tile<EPI>(g, BN, blockIdx.z);
+}
+
+// The weight gradients of several layers in one launch: gridDim.z = layers x splits.  Their shapes may
+// differ; blocks past a layer's rows or columns return at once.
+struct GemmBatch {
+  GemmArgs g[kMaxLayers];
+  int splits;
+};
+
+__global__ void __launch_bounds__(kGtThreads, 1) gemm_batch_tc(const __grid_constant__ GemmBatch b, int BN) {
+  gemm_tc_tile<EPI_PARTIAL>(b.g[blockIdx.z / b.splits], BN, blockIdx.z % b.splits);
 }
 
 // Adam on the FP32 parameters, then the padded BF16 copies W [out_pad][in_pad] and W^T [in_pad][out_pad].
@@ -867,7 +892,8 @@ struct BdMlp {
   std::vector<float*> Z;
   std::vector<bf16*> A, At, dZ, dZt;
   float *Y = nullptr, *part = nullptr, *loss_part = nullptr, *loss_tmp = nullptr;
-  long long part_stride = 0;
+  long long part_bytes = 0;
+  bool batch_attr = false;
   int inference = 1;  // 1: tcgen05 kernel when the shape allows, 0: mma.sync GEMM chain
   int gemm_tc = 1;    // GEMMs of training and of the GEMM chain: 1 tcgen05 (gemm_nt_tc), 0 mma.sync
   bool gt_attr = false;
@@ -959,6 +985,25 @@ int gemm(BdMlp* m, const GemmArgs& g, int splits, cudaStream_t s) {
   return launch_gemm<128, 32, 4, 2, EPI>(m, g, splits, s);
 }
 
+// The split partials of `cnt` layers' weight gradients in one launch (n and the split length are multiples
+// of 32, the padded widths of 32).  64-wide tiles: two CTAs per SM hide each other's loads.
+int gemm_batch(BdMlp* m, const GemmBatch& b, int cnt, int max_m, int max_n, int splits, cudaStream_t s) {
+  const int BN = std::min(max_n, 64);
+  if (!m->batch_attr) {
+    MCK(m, cudaFuncSetAttribute(gemm_batch_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, gt_smem_bytes(64)));
+    m->batch_attr = true;
+  }
+  gemm_batch_tc<<<dim3((max_n + BN - 1) / BN, (max_m + 127) / 128, cnt * splits), kGtThreads, gt_smem_bytes(BN), s>>>(b,
+                                                                                                               BN);
+  MCK(m, cudaGetLastError());
+  return BD_OK;
+}
+
+constexpr long long kPartBytes = 128ll << 20;  // split partials of the weight gradients kept at once
+
+// Splits of the batch in the weight gradients.
+int train_splits(int n) { return std::max(1, std::min(64, n / 512)); }
+
 int ensure_train(BdMlp* m, int n) {
   if (n <= m->train_cap) return BD_OK;
   if (m->train_graph) {  // it holds the old buffers
@@ -997,10 +1042,15 @@ int ensure_train(BdMlp* m, int n) {
   if (!(m->Y = (float*)get((size_t)n * op * 4))) return rc;
   if (!(m->dY = (bf16*)get((size_t)n * op * 2))) return rc;
   if (!(m->dYt = (bf16*)get((size_t)n * op * 2))) return rc;
-  int maxw = 0;
-  for (int l = 0; l < nl; ++l) maxw = std::max(maxw, L.out_pad[l] * L.in_pad[l]);
-  m->part_stride = maxw;
-  if (!(m->part = (float*)get((size_t)64 * maxw * 4))) return rc;
+  // split partials of the weight gradients: every layer's, up to kPartBytes; one layer's at least
+  long long all = 0, one = 0;
+  for (int l = 0; l < nl; ++l) {
+    all += (long long)L.out_pad[l] * L.in_pad[l];
+    one = std::max(one, (long long)L.out_pad[l] * L.in_pad[l]);
+  }
+  // a smaller batch may round to one split more than its share
+  m->part_bytes = std::max(one * 64 * 4, std::min(all * (train_splits(n) + 1) * 4, kPartBytes));
+  if (!(m->part = (float*)get((size_t)m->part_bytes))) return rc;
   if (!(m->loss_part = (float*)get((size_t)m->n_sm * 16 * 4))) return rc;
   if (!(m->loss_tmp = (float*)get(4))) return rc;
   m->train_cap = n;
@@ -1129,42 +1179,13 @@ int backward(BdMlp* m, int member, int n, const float* X, const float* T, float*
   loss_finish_kernel<<<1, 32, 0, s>>>(m->loss_part, nb, (float)n * (float)m->d.out_dim, loss ? loss : m->loss_tmp,
                                      trace, trace ? m->data_step : nullptr);
   MCK(m, cudaGetLastError());
-  // split-K of the weight gradients: 512 rows per split (16 at batch 8192) keep every SM busy
-  // while halving the partials that grad_reduce_kernel reads back
-  const int splits = std::max(1, std::min(64, n / 512));
-  const int kps = round_up((n + splits - 1) / splits, kBK);
-  for (int l = nl - 1; l >= 0; --l) {
-    const bf16* dZ = l == nl - 1 ? m->dY : m->dZ[l];
-    const bf16* dZt = l == nl - 1 ? m->dYt : m->dZt[l];
-    const bf16* Ain_t = l == 0 ? m->Xt : m->At[l - 1];
-    // dW_l = dZ_l^T A_{l-1}: M = out_pad, N = in_pad, K = n
-    GemmArgs g{};
-    g.M = L.out_pad[l];
-    g.N = L.in_pad[l];
-    g.K = n;
-    g.A = dZt;
-    g.lda = n;
-    g.B = Ain_t;
-    g.ldb = n;
-    g.k_per_split = kps;
-    g.C = m->part;
-    g.ldc = L.in_pad[l];
-    g.split_stride = m->part_stride;
-    const int used = (n + kps - 1) / kps;
-    if ((rc = gemm<EPI_PARTIAL>(m, g, used, s))) return rc;
-    const int tot = L.out_real[l] * L.in_real[l];
-    grad_reduce_kernel<<<grid_for(m, tot), 256, 0, s>>>(m->part, used, m->part_stride, L.in_pad[l], L.out_real[l],
-                                                         L.in_real[l], w.grad + L.w_off[l]);
-    MCK(m, cudaGetLastError());
-    bias_grad_kernel<<<L.out_real[l], 256, 0, s>>>(dZt, n, n, L.out_real[l], w.grad + L.b_off[l]);
-    MCK(m, cudaGetLastError());
-    if (l == 0) break;
-    // dZ_{l-1} = (dZ_l W_l) * SiLU'(Z_{l-1}): M = n, N = in_pad (hidden), K = out_pad
-    GemmArgs b{};
+  // dZ of every hidden layer, last to first: dZ_{l-1} = (dZ_l W_l) * SiLU'(Z_{l-1})
+  for (int l = nl - 1; l > 0; --l) {
+    GemmArgs b{};  // M = n, N = in_pad (hidden), K = out_pad
     b.M = n;
     b.N = L.in_pad[l];
     b.K = L.out_pad[l];
-    b.A = dZ;
+    b.A = l == nl - 1 ? m->dY : m->dZ[l];
     b.lda = L.out_pad[l];
     b.B = w.Wt + L.wb_off[l];
     b.ldb = L.out_pad[l];
@@ -1176,6 +1197,51 @@ int backward(BdMlp* m, int member, int n, const float* X, const float* T, float*
     b.Ot = m->dZt[l - 1];
     b.ldot = n;
     if ((rc = gemm<EPI_HIDDEN_BWD>(m, b, 1, s))) return rc;
+  }
+  // Weight and bias gradients: dW_l = dZ_l^T A_{l-1} (M = out_pad, N = in_pad, K = n) in split partials,
+  // 512 rows per split (16 at batch 8192: every SM busy), then one kernel of sums.  They depend only on the
+  // chain above, so the layers whose partials fit the buffer share both launches (all of them up to
+  // kPartBytes); one launch of 128 blocks per layer, with two small kernels each, took 120 us of 337.
+  const int splits = train_splits(n);
+  const int kps = round_up((n + splits - 1) / splits, kBK), used = (n + kps - 1) / kps;
+  for (int hi = nl - 1; hi >= 0;) {
+    GemmBatch gb{};
+    GradBatch fb{};
+    gb.splits = used;
+    fb.n = n;
+    int cnt = 0, max_m = 0, max_n = 0, max_tot = 0, max_out = 0;
+    long long at = 0;
+    for (; hi >= 0; --hi, ++cnt) {
+      const int l = hi;
+      const long long size = (long long)L.out_pad[l] * L.in_pad[l];
+      if (cnt > 0 && (at + size * used) * 4 > m->part_bytes) break;
+      GemmArgs& g = gb.g[cnt];
+      g.M = L.out_pad[l];
+      g.N = L.in_pad[l];
+      g.K = n;
+      g.A = l == nl - 1 ? m->dYt : m->dZt[l];
+      g.lda = n;
+      g.B = l == 0 ? m->Xt : m->At[l - 1];
+      g.ldb = n;
+      g.k_per_split = kps;
+      g.C = m->part + at;
+      g.ldc = L.in_pad[l];
+      g.split_stride = size;
+      fb.l[cnt] = {g.C, size, used, g.ldc, L.out_real[l], L.in_real[l], g.A, w.grad + L.w_off[l], w.grad + L.b_off[l]};
+      at += size * used;
+      max_m = std::max(max_m, g.M);
+      max_n = std::max(max_n, g.N);
+      max_tot = std::max(max_tot, L.out_real[l] * L.in_real[l]);
+      max_out = std::max(max_out, L.out_real[l]);
+    }
+    if (m->gemm_tc) {
+      if ((rc = gemm_batch(m, gb, cnt, max_m, max_n, used, s))) return rc;
+    } else {
+      for (int i = 0; i < cnt; ++i)
+        if ((rc = gemm<EPI_PARTIAL>(m, gb.g[i], used, s))) return rc;
+    }
+    grad_finish_kernel<<<dim3(max_out + grid_for(m, max_tot), cnt), 256, 0, s>>>(fb);
+    MCK(m, cudaGetLastError());
   }
   return BD_OK;
 }
