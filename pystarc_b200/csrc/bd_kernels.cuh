@@ -15,9 +15,13 @@ __device__ __forceinline__ double gsum(double v, unsigned m) {
 
 template <int G>
 __device__ __forceinline__ unsigned gsumu(unsigned v, unsigned m) {
+  if constexpr (G == 32) {
+    return __reduce_add_sync(m, v);  // one instruction for whole numbers
+  } else {
 #pragma unroll
-  for (int o = G / 2; o > 0; o >>= 1) v += __shfl_xor_sync(m, v, o, G);
-  return v;
+    for (int o = G / 2; o > 0; o >>= 1) v += __shfl_xor_sync(m, v, o, G);
+    return v;
+  }
 }
 
 template <int G>

@@ -88,7 +88,7 @@ __global__ void __launch_bounds__(256, 2) pose_block_kernel(const __grid_constan
     __syncthreads();
     if (rev) {
       unsigned nr = 0;
-      group_reverse_born<FT, TORQUE>(S, src, lane, warp, 8, 1, sh.rev, TORQUE ? sh.rev + 8 * kSplitBuf<FT> : sh.rev,
+      group_reverse_born<FT, TORQUE, true>(S, src, lane, warp, 8, 1, sh.rev, TORQUE ? sh.rev + 8 * kSplitBuf<FT> : sh.rev,
                                      cnts, r, u, nr);
       const double* sum = warp == 0 ? r : u;
       if (warp < 2) {

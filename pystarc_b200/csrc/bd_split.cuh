@@ -74,14 +74,20 @@ struct OneTab {
   }
 };
 
-// Append the lanes with `want` to a list whose length is *len: one atomic per warp.
-__device__ __forceinline__ void warp_append(int* list, int* len, bool want, int value, int lane) {
-  const unsigned m = __ballot_sync(0xffffffffu, want);
-  if (!m) return;
-  int at = 0;
-  if (lane == __ffs(m) - 1) at = atomicAdd(len, __popc(m));
-  at = __shfl_sync(0xffffffffu, at, __ffs(m) - 1);
-  if (want) list[at + __popc(m & ((1u << lane) - 1u))] = value;
+// Append the lanes with `eval` to flist and those with `rev` (which have `eval` too) to rlist: one
+// atomic per warp on the pair of their lengths.
+__device__ __forceinline__ void warp_append(const SplitBuf& U, int set, bool eval, bool rev, int slot, int lane) {
+  const unsigned me = __ballot_sync(0xffffffffu, eval), mr = __ballot_sync(0xffffffffu, rev);
+  if (!me) return;
+  unsigned long long at = 0;
+  const int leader = __ffs(me) - 1;
+  if (lane == leader)
+    at = atomicAdd(reinterpret_cast<unsigned long long*>(U.cnt + set),
+                   (unsigned long long)__popc(mr) << 32 | (unsigned long long)__popc(me));
+  at = __shfl_sync(0xffffffffu, at, leader);
+  const unsigned below = (1u << lane) - 1u;
+  if (eval) U.flist[(int)(at & 0xffffffffull) + __popc(me & below)] = slot;
+  if (rev) U.rlist[(int)(at >> 32) + __popc(mr & below)] = slot;
 }
 
 // END: finish the step begun by the previous launch of this kernel; BEGIN: begin the next one.
@@ -115,22 +121,27 @@ __global__ void __launch_bounds__(kStepBlock, 4) split_step_kernel(const __grid_
     if (END) {
       const DevSystem& S = T.sys(k);
       const DevSim& P = T.sim(k);
-      const int mode = own ? (int)U.mode[slot] : 0;
-      const bool need = mode != 0;
-      double R[9] = {1, 0, 0, 0, 1, 0, 0, 0, 1}, r = 0;
-      double F[3] = {0, 0, 0}, Tq[3] = {0, 0, 0};
-      if (need) {
-        quat_to_rot(tr.q, R);
-        r = norm3(tr.c[0], tr.c[1], tr.c[2]);
+      // everything the slot may need is loaded at once, before its mode is known
+      int mode = 0;
+      double F[3] = {0, 0, 0}, Tq[3] = {0, 0, 0}, rv[6] = {0, 0, 0, 0, 0, 0};
+      if (own) {
+        mode = (int)U.mode[slot];
 #pragma unroll
         for (int i = 0; i < 3; ++i) {
           F[i] = U.F[3 * slot + i];
           Tq[i] = U.T[3 * slot + i];
+          rv[i] = U.rv[6 * slot + i];
+          rv[3 + i] = U.rv[6 * slot + 3 + i];
         }
+      }
+      const bool need = mode != 0;
+      double R[9] = {1, 0, 0, 0, 1, 0, 0, 0, 1}, r = 0;
+      if (need) {
+        quat_to_rot(tr.q, R);
+        r = norm3(tr.c[0], tr.c[1], tr.c[2]);
         if (mode == 3) {
           // the reverse-Born force on the receptor, rotated to the lab frame, acts on the ligand
           // with the opposite sign
-          const double* rv = U.rv + 6 * slot;
 #pragma unroll
           for (int i = 0; i < 3; ++i) F[i] = F[i] - (R[3 * i] * rv[0] + R[3 * i + 1] * rv[1] + R[3 * i + 2] * rv[2]);
           if (TORQUE) {
@@ -198,8 +209,7 @@ __global__ void __launch_bounds__(kStepBlock, 4) split_step_kernel(const __grid_
       const bool reuse = need && keep && tr.rets == rets0;
       const bool eval = need && !reuse;
       const bool rev = eval && S.born_rev && r - S.rec_max_r < S.lig_born_rho;
-      warp_append(U.flist, U.cnt + 4 * set, eval, slot, lane);
-      warp_append(U.rlist, U.cnt + 4 * set + 1, rev, slot, lane);
+      warp_append(U, 4 * set, eval, rev, slot, lane);
       if (run && st != ST_RUNNING) {
         tr.status = st;
         P.out_status[tr.id] = (int8_t)st;
@@ -468,15 +478,19 @@ struct RevPose {
     cz = (FT)c[2];
   }
 
-  // Chunk k's bounding sphere reaches the box.
-  __device__ __forceinline__ bool hits(const DevSystem& S, int k) const {
-    if (k >= S.n_chunks) return false;
+  // Chunk k's bounding sphere; past the last chunk one that reaches nothing.
+  static __device__ __forceinline__ V4 sphere(const DevSystem& S, int k) {
+    if (k >= S.n_chunks) return Vec4<FT>::make(0, 0, 0, (FT)-1);
+    if constexpr (sizeof(FT) == 4) return S.chunks_f[k];
+    else return S.chunks[k];
+  }
+
+  // A chunk's bounding sphere reaches the box.
+  __device__ __forceinline__ bool reaches(const DevSystem& S, const V4& sp) const {
+    if (sp.w < (FT)0) return false;
     const DevGrid& g = S.lig_born;
     const FT lox = in<FT>(g.lox, g.loxf), loy = in<FT>(g.loy, g.loyf), loz = in<FT>(g.loz, g.lozf);
     const FT hix = in<FT>(g.hix, g.hixf), hiy = in<FT>(g.hiy, g.hiyf), hiz = in<FT>(g.hiz, g.hizf);
-    V4 sp;
-    if constexpr (sizeof(FT) == 4) sp = S.chunks_f[k];
-    else sp = S.chunks[k];
     const FT d0 = (FT)sp.x - cx, d1 = (FT)sp.y - cy, d2 = (FT)sp.z - cz;
     const FT l0 = Rt[0] * d0 + Rt[3] * d1 + Rt[6] * d2;
     const FT l1 = Rt[1] * d0 + Rt[4] * d1 + Rt[7] * d2;
@@ -554,7 +568,7 @@ __device__ __forceinline__ void lean_reverse_born(const DevSystem& S, const SRC&
             done = true;
             break;
           }
-          hits = __ballot_sync(FULL, pose.hits(S, k0 + lane));
+          hits = __ballot_sync(FULL, pose.reaches(S, pose.sphere(S, k0 + lane)));
           k0 += 32;
           continue;
         }
@@ -623,7 +637,7 @@ __device__ __forceinline__ void lean_reverse_born(const DevSystem& S, const SRC&
 // coefficient and gradient (it is `buf` itself when the positions are not needed again);
 // cnt: two rows of W counts.  Every warp of the group takes the same path (the culls and counts
 // it depends on are the same on each), so the group's barriers match.
-template <typename FT, bool TORQUE, class SRC>
+template <typename FT, bool TORQUE, bool AHEAD, class SRC>
 __device__ __forceinline__ void group_reverse_born(const DevSystem& S, const SRC& src, int lane, int gw, int W, int bar, typename Vec4<FT>::type* buf,
                                                    typename Vec4<FT>::type* val, int* cnt, double r[3], double u[3],
                                                    unsigned& nr) {
@@ -679,9 +693,15 @@ __device__ __forceinline__ void group_reverse_born(const DevSystem& S, const SRC
     // lane l keeps the hit mask of chunks c0 + 32 l .. + 31
     unsigned mine = 0;
     const int n_mask = min(32, (S.n_chunks - c0 + 31) / 32);
-    for (int l = 0; l < n_mask; ++l) {
-      const unsigned m = __ballot_sync(FULL, pose.hits(S, c0 + 32 * l + lane));
-      if (lane == l) mine = m;
+    for (int l = 0; l < n_mask; l += 4) {  // four loads in flight
+      V4 sp[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) sp[j] = pose.sphere(S, c0 + 32 * (l + j) + lane);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const unsigned m = __ballot_sync(FULL, pose.reaches(S, sp[j]));
+        if (lane == l + j) mine = m;
+      }
     }
     int before = __popc(mine);  // exclusive prefix of the hit counts
 #pragma unroll
@@ -691,32 +711,48 @@ __device__ __forceinline__ void group_reverse_born(const DevSystem& S, const SRC
     }
     const int H = __shfl_sync(FULL, before, 31);
     before -= __popc(mine);
+    // the chunk of hit h: its mask's lane, then the bit with that many hits below it
+    auto chunk_of = [&](int h) {
+      const unsigned has = __ballot_sync(FULL, before <= h && h < before + __popc(mine));
+      const int ml = __ffs(has) - 1;
+      const unsigned m = __shfl_sync(FULL, mine, ml);
+      const int nth = h - __shfl_sync(FULL, before, ml);
+      const unsigned bit = __ballot_sync(FULL, ((m >> lane) & 1u) && __popc(m & ((1u << lane) - 1u)) == nth);
+      return c0 + 32 * ml + __ffs(bit) - 1;
+    };
+    int kk = -1;
+    V4 at{};
+    if (AHEAD && gw < H) {
+      kk = chunk_of(gw);
+      at = pose.atom(S, kk * BD_CHUNK + lane);
+    }
     for (int h0 = 0; h0 < H; h0 += W) {
-      const int h = h0 + gw;
-      V4 ent{};
-      bool cand = false;
-      if (h < H) {
-        // the chunk of hit h: its mask's lane, then the bit with that many hits below it
-        const unsigned has = __ballot_sync(FULL, before <= h && h < before + __popc(mine));
-        const int ml = __ffs(has) - 1;
-        const unsigned m = __shfl_sync(FULL, mine, ml);
-        const int nth = h - __shfl_sync(FULL, before, ml);
-        const unsigned at =
-            __ballot_sync(FULL, ((m >> lane) & 1u) && __popc(m & ((1u << lane) - 1u)) == nth);
-        const int idx = (c0 + 32 * ml + __ffs(at) - 1) * BD_CHUNK + lane;
-        cand = pose.candidate(S, src, idx, pose.atom(S, idx), ent);
+      // AHEAD: the warp's next chunk loads while this one's atoms are tested
+      int kn = -1;
+      V4 an = at, ent{};
+      if (!AHEAD) {
+        kk = h0 + gw < H ? chunk_of(h0 + gw) : -1;
+        if (kk >= 0) at = pose.atom(S, kk * BD_CHUNK + lane);
+      } else if (h0 + W + gw < H) {
+        kn = chunk_of(h0 + W + gw);
+        an = pose.atom(S, kn * BD_CHUNK + lane);
+      }
+      const bool cand = kk >= 0 && pose.candidate(S, src, kk * BD_CHUNK + lane, at, ent);
+      if (AHEAD) {
+        at = an;
+        kk = kn;
       }
       const unsigned m = __ballot_sync(FULL, cand);
       if (lane == 0) cnt[flip * 8 + gw] = __popc(m);
       group_sync(bar, 32 * W);
-      int at = head, total = 0;
+      int place = head, total = 0;
       for (int w = 0; w < W; ++w) {
         const int k = cnt[flip * 8 + w];
-        if (w < gw) at += k;
+        if (w < gw) place += k;
         total += k;
       }
       flip ^= 1;
-      if (cand) buf[at + __popc(m & ((1u << lane) - 1u))] = ent;
+      if (cand) buf[place + __popc(m & ((1u << lane) - 1u))] = ent;
       head += total;
       if (head > (kSplitBuf<FT> - 32) * W) {  // no room for another round
         const int n = head & ~31, rem = head - n;
@@ -770,7 +806,7 @@ __global__ void __launch_bounds__(256, sizeof(FT) == 4 ? 4 : 2) split_rev_kernel
       lean_reverse_born<FT, TORQUE, sizeof(FT) == 8>(S, SlotSrc{B, slot}, lane, bufs[warp], r, u, nr);
     } else {
       V4* buf = bufs[grp * W];
-      group_reverse_born<FT, TORQUE>(S, SlotSrc{B, slot}, lane, gw, W, 1 + grp, buf, TORQUE ? vals[grp * W] : buf,
+      group_reverse_born<FT, TORQUE, sizeof(FT) == 8>(S, SlotSrc{B, slot}, lane, gw, W, 1 + grp, buf, TORQUE ? vals[grp * W] : buf,
                                      cnts[grp], r, u, nr);
     }
     if (gw == 0) {
