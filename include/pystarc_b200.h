@@ -220,9 +220,10 @@ int bd_sim_restore(BdHandle* h, const double* c, const double* q, const int32_t*
  * trajectory's whole step) or BD_GROUP_WARP (each lane owns one trajectory's step logic and
  * the warp sweeps each trajectory's atoms together; BD_GROUP_WARP_CAPPED is the same with
  * registers capped at 128 per thread), or BD_GROUP_SPLIT (each BD step as three kernels: the
- * ligand-atom forces, Born direction 2 in a kernel capped at 64 registers, then the rest of the
- * step; the same trajectories as BD_GROUP_WARP), and threads per block (multiple of 32, <= 256).
- * Set by the autotuner; 0 keeps the current value. */
+ * scalar part, which lists the poses that need forces, the ligand-atom forces and Born direction 2
+ * of the listed poses; the same trajectories as BD_GROUP_WARP; the default wherever there is a
+ * receptor to sweep), and threads per block (multiple of 32, <= 256; the split step's kernels have
+ * their own).  Set by the autotuner; 0 keeps the current value. */
 enum { BD_GROUP_WARP = 64, BD_GROUP_WARP_CAPPED = 65, BD_GROUP_SPLIT = 66 };
 int bd_set_launch(BdHandle* h, int group, int block_threads);
 int bd_get_launch(BdHandle* h, int* group, int* block_threads, int* grid_blocks);
@@ -398,7 +399,7 @@ int bd_sim_surrogate_counters(BdHandle* h, uint64_t* out);
 /* ---- Heterogeneous batch -----------------------------------------------------------------
  * No reference counterpart (the reference runs one system per process).  Trajectories of n
  * configured handles (each with its own grids, atoms, reactions and BdSimParams; the same
- * precision and torque mode) share one slot pool and one persistent launch; a slot holds the
+ * precision and torque mode) share one slot pool and the split step's launches; a slot holds the
  * trajectory's index in the concatenation of the systems' ranges.  Outcomes land in each
  * handle's own arrays (read them with bd_sim_outcomes); the counters are summed over the
  * systems.  The handles must stay configured and unchanged while the batch exists.  Noise keys

@@ -8,8 +8,8 @@ The tuned "tile shapes" of the stepper:
   G = 64 / 65           each lane owns one trajectory's step logic and the warp sweeps each
                         trajectory's ligand atoms 32 at a time (65: registers capped at 128
                         per thread for more resident warps)
-  G = 66                the split step: ligand atoms as in 64, Born direction 2 in a kernel of
-                        its own capped at 64 registers (twice the resident warps)
+  G = 66                the split step: a scalar kernel that lists the poses, then the ligand atoms
+                        and Born direction 2 of the listed poses in a kernel each, a warp per pose
 * trajectories per CTA -- threads per block (128 or 256) divided by the lanes per trajectory;
 * the receptor tile of Born direction 2 -- how the ligand Born grid is read: float4 windows of
   4 z-nodes (8 loads per stencil) or 2x2x2 node cubes (4 loads, 8x the grid's memory).

@@ -121,9 +121,18 @@ int dev_alloc(BdHandle* h, std::vector<void*>& list, void** p, size_t bytes) {
   return BD_OK;
 }
 
+// Free the buffers that no sim_alloc has taken since they were marked unused.
+void free_unused(BdHandle* h) {
+  auto& v = h->sim_blocks;
+  for (auto& b : v)
+    if (!b.used) cudaFree(b.p);
+  v.erase(std::remove_if(v.begin(), v.end(), [](const BdHandle::SimBlock& b) { return !b.used; }), v.end());
+}
+
 // A device buffer of the configured run.  A run with the sizes of the one before it takes that
 // one's buffers: freeing and allocating the pool again took 6 ms a run for two spheres (100,000
-// trajectories).  bd_sim_configure gives back what the new run did not take.
+// trajectories).  bd_sim_configure gives back what the new run did not take; a run that does not
+// fit beside them gives them back first.
 int sim_alloc(BdHandle* h, void** p, size_t bytes) {
   if (!bytes) bytes = 16;
   for (auto& b : h->sim_blocks)
@@ -132,17 +141,15 @@ int sim_alloc(BdHandle* h, void** p, size_t bytes) {
       *p = b.p;
       return BD_OK;
     }
-  CK(h, cudaMalloc(p, bytes));
+  cudaError_t e = cudaMalloc(p, bytes);
+  if (e == cudaErrorMemoryAllocation) {
+    cudaGetLastError();
+    free_unused(h);
+    e = cudaMalloc(p, bytes);
+  }
+  CK(h, e);
   h->sim_blocks.push_back({*p, bytes, true});
   return BD_OK;
-}
-
-// Free the buffers that no sim_alloc has taken since they were marked unused.
-void free_unused(BdHandle* h) {
-  auto& v = h->sim_blocks;
-  for (auto& b : v)
-    if (!b.used) cudaFree(b.p);
-  v.erase(std::remove_if(v.begin(), v.end(), [](const BdHandle::SimBlock& b) { return !b.used; }), v.end());
 }
 
 void free_list(std::vector<void*>& list) {

@@ -1,4 +1,4 @@
-"""Heterogeneous batch: several receptor-ligand systems in one persistent launch.
+"""Heterogeneous batch: several receptor-ligand systems in one pool and its launches.
 
 No reference counterpart: the reference runs one system per process.  Each
 system is a configured ``B200BatchSimulator`` (its own engine, grids, atoms,
