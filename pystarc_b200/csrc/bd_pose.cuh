@@ -142,7 +142,7 @@ __global__ void __launch_bounds__(256, 2) pose_fwd_kernel(const __grid_constant_
 }
 
 template <typename FT, bool TORQUE>
-__global__ void __launch_bounds__(256, sizeof(FT) == 4 ? 4 : 2) pose_rev_kernel(const __grid_constant__ DevSystem S,
+__global__ void __launch_bounds__(256, sizeof(FT) == 4 ? (TORQUE ? 3 : 4) : 2) pose_rev_kernel(const __grid_constant__ DevSystem S,
                                                                                const __grid_constant__ PoseBatch P) {
   using V4 = typename Vec4<FT>::type;
   __shared__ V4 bufs[8][kSplitBuf<FT>];

@@ -781,10 +781,13 @@ __device__ __forceinline__ int rev_warps(int n, int n_warps) {
   return n * 4 <= n_warps ? 8 : n * 2 <= n_warps ? 4 : n <= n_warps ? 2 : 1;
 }
 
-// FP32: capped at 64 registers, 32 warps per SM.  FP64: at 128; the cap of 80 spills 388 bytes and
-// measured slower (30,011 FP64 trajectories: 147 against 136 ms of GPU time).
+// FP32 without torque: capped at 64 registers, 32 warps per SM (at 80 and 24 warps 150,000 trajectories
+// take 330 instead of 312 ms of GPU time).  With torque that cap spills 164 bytes: at 80 it spills none,
+// and 8,000 trajectories take 107 instead of 121 ms, 6,000 protein pairs 106 instead of 113, 150,000
+// (768 steps) 249 instead of 252.  FP64: at 128; a cap of 80 spills 450 bytes and is slower (30,011
+// trajectories 114 -> 128 ms).
 template <typename FT, bool TORQUE, class TAB>
-__global__ void __launch_bounds__(256, sizeof(FT) == 4 ? 4 : 2) split_rev_kernel(const __grid_constant__ TAB T,
+__global__ void __launch_bounds__(256, sizeof(FT) == 4 ? (TORQUE ? 3 : 4) : 2) split_rev_kernel(const __grid_constant__ TAB T,
                                                                                 SlotBuf B, SplitBuf U, int set) {
   using V4 = typename Vec4<FT>::type;
   __shared__ V4 bufs[8][kSplitBuf<FT>];
