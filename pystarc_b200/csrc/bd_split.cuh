@@ -418,8 +418,14 @@ __global__ void __launch_bounds__(256, 2) split_fwd_kernel(const __grid_constant
         for (int i = 0; i < 9; ++i) R[i] = __shfl_sync(FULL, pose.R[i], src);
         const int to = __shfl_sync(FULL, slot, src);
         const DevSystem& S = T.sys(__shfl_sync(FULL, sys, src));
-        quarter_forces<FT, TORQUE>(S, c, R, lane & 7, f, t, cnt);
-        if (base + src < n) store_force(U, to, lane & 7, f, t);
+        Counts mine{0, 0, 0};
+        quarter_forces<FT, TORQUE>(S, c, R, lane & 7, f, t, mine);
+        // past the end of the list the lanes repeat a pose, for the shuffles' sake
+        if (base + src < n) {
+          store_force(U, to, lane & 7, f, t);
+          cnt.grid += mine.grid;
+          cnt.ff += mine.ff;
+        }
       }
     }
   } else if (const int W = T.large_ligands() ? fwd_warps(n, n_warps) : 1; W > 1) {
