@@ -317,7 +317,8 @@ class B200BatchSimulator:
         return self.id_offset + (0 if self._shard is None else self._shard[2])
 
     # ------------------------------------------------------------------
-    def _setup(self):
+    def _setup(self, slots=None):
+        """Configure the device for this run; ``slots`` replaces the pool size the caller asked for."""
         p = self.params
         D_t = float(self.mob.relative_translational_diffusion())
         D_r = float(self.mob.relative_rotational_diffusion())
@@ -384,7 +385,7 @@ class B200BatchSimulator:
         sp.r_hydro_lig = r_h_lig
         sp.precision = {"fp64": _lib.PREC_FP64, "mixed": _lib.PREC_MIXED}[self.precision]
         sp.torque_mode = {"zero": _lib.TORQUE_ZERO, "centroid": _lib.TORQUE_CENTROID}[self.torque_mode]
-        sp.slots = self.slots
+        sp.slots = self.slots if slots is None else int(slots)
         sp.id_offset = self._offset
         sp.stats = int(self.stats)
         sp.save_interval = self._save_interval
@@ -552,18 +553,27 @@ class B200BatchSimulator:
         h = self.engine.handle
         cap = _lib.C.c_int32()
         h.call("bd_sim_capacity", _lib.C.byref(cap))
-        if int(d["cap"]) != cap.value:
-            raise ValueError(f"{path}: slot capacity {int(d['cap'])} != {cap.value}")
+        saved = int(d["cap"])
+        # the default capacity follows from the stepper's resident blocks and so changes with its kernels:
+        # a run that asked for no pool size of its own takes the checkpoint's
+        if saved != cap.value and (self.slots > 0 or not 0 < saved <= self._n_run):
+            raise ValueError(f"{path}: slot capacity {saved} != {cap.value}")
         arr = {}
         for k in d.files:  # each NpzFile lookup reads the member again: one lookup per key
             v = d[k]
             arr[k] = np.ascontiguousarray(v) if v.ndim else v[()]
+        for k, width in (("c", 3), ("q", 4), ("traj", 1), ("steps", 1), ("rets", 1), ("status", 1)):
+            if arr[k].size != width * saved:
+                raise ValueError(f"{path}: {arr[k].size} values of {k} for {saved} slots")
+        if saved != cap.value:
+            self._setup(slots=saved)
+            h.call("bd_sim_reset", None)
         h.call("bd_sim_restore", _lib.ptr(arr["c"]), _lib.ptr(arr["q"]), _lib.ptr(arr["traj"], _lib.C.c_int32),
                _lib.ptr(arr["steps"], _lib.C.c_int32), _lib.ptr(arr["rets"], _lib.C.c_int32),
                _lib.ptr(arr["status"], _lib.C.c_int8), int(arr["n_live"]), _lib.ptr(arr["counters"], _lib.C.c_uint64),
                _lib.ptr(arr["out_status"], _lib.C.c_int8), _lib.ptr(arr["out_steps"], _lib.C.c_int32),
                _lib.ptr(arr["out_returns"], _lib.C.c_int32))
-        state = np.ascontiguousarray(arr["state"], dtype=np.int8) if "state" in arr else np.zeros(cap.value, np.int8)
+        state = np.ascontiguousarray(arr["state"], dtype=np.int8) if "state" in arr else np.zeros(saved, np.int8)
         h.call("bd_sim_set_states", _lib.ptr(state, _lib.C.c_int8))
 
     # ------------------------------------------------------------------
