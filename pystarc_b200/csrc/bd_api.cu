@@ -1444,6 +1444,7 @@ int ensure_split_buffers(BdHandle* h) {
 // step do not depend on each other: the sweep is captured on a branch of its own.
 struct SplitPlan {
   const SplitKernels* kn;
+  void* fwd;       // kn->fwd or kn->fwd_long (split_fwd)
   void* tab;       // OneTab or MultiTab (copied at capture)
   SplitBuf U;
   bool rev;        // some system has Born direction 2
@@ -1473,7 +1474,7 @@ cudaError_t enqueue_split_steps(const SplitPlan& p, SlotBuf src, SlotBuf dst, co
           !ok(cudaEventRecord(p.join, p.side)))
         return e;
     }
-    if (!ok(cudaLaunchKernel(p.kn->fwd, dim3(p.b_fwd), dim3(256), f_args, 0, s))) return e;
+    if (!ok(cudaLaunchKernel(p.fwd, dim3(p.b_fwd), dim3(256), f_args, 0, s))) return e;
     if (p.rev && !ok(cudaStreamWaitEvent(s, p.join, 0))) return e;
   }
   compact_kernel<<<p.n_sm * 4, 256, 0, s>>>(src, dst, live, p.ctr);
@@ -1482,13 +1483,20 @@ cudaError_t enqueue_split_steps(const SplitPlan& p, SlotBuf src, SlotBuf dst, co
   return cudaGetLastError();
 }
 
+// The ligand-atom kernel of a pool of `cap` slots: the one that takes several list entries a turn where a
+// list can be that long, unless four poses share a warp (mixed precision, small ligands).
+void* split_fwd(const SplitKernels& kn, int cap, int warps, int precision, bool small) {
+  return cap >= 2 * kLongTurns * warps && !(precision == BD_PREC_MIXED && small) ? kn.fwd_long : kn.fwd;
+}
+
 int enqueue_split_launch(BdHandle* h, int K, cudaStream_t s, int cur) {
   const SplitKernels& kn = table_for(h->sp.precision, h->sp.torque_mode).split;
   OneTab T{h->S, h->P};
-  SplitPlan p{&kn, &T, h->split_buf, h->S.born_rev != 0, stepper_smem(h->S, h->P, kn.mid)};
+  SplitPlan p{&kn, kn.fwd, &T, h->split_buf, h->S.born_rev != 0, stepper_smem(h->S, h->P, kn.mid)};
   stepper_smem(h->S, h->P, kn.last);
   p.b_step = persistent_blocks(h, kn.mid, kStepBlock, p.smem);
   p.b_fwd = persistent_blocks(h, kn.fwd, 256);
+  p.fwd = split_fwd(kn, h->buf[0].cap, 8 * p.b_fwd, h->sp.precision, h->S.n_lig <= 32 && !h->S.wca);
   p.b_rev = persistent_blocks(h, kn.rev, 256);
   p.side = h->side;
   p.fork = h->fork;
@@ -1963,9 +1971,10 @@ int multi_graphs(BdMulti* m, int K) {
     return per_sm * m->n_sm;
   };
   MultiTab T = m->T;
-  SplitPlan p{&kn, &T, m->split, m->rev, 0};
+  SplitPlan p{&kn, kn.fwd, &T, m->split, m->rev, 0};
   p.b_step = blocks(kn.mid, kStepBlock);
   p.b_fwd = blocks(kn.fwd, 256);
+  p.fwd = split_fwd(kn, m->cap, 8 * p.b_fwd, m->precision, m->T.small);
   p.b_rev = blocks(kn.rev, 256);
   p.side = m->side;
   p.fork = m->fork;
@@ -2028,6 +2037,7 @@ int bd_multi_create(BdHandle* const* handles, int n, BdMulti** out) {
     sim[i].stats = 0;
     base[i + 1] = base[i] + h->P.n_traj;
     m->rev = m->rev || h->S.born_rev;
+    m->T.largest = std::max(m->T.largest, h->S.n_lig);
     m->T.small = (i == 0 || m->T.small) && h->S.n_lig <= 32 && !h->S.wca;
     m->T.large = (i == 0 || m->T.large) && h->S.n_lig >= 128 && !h->S.wca;
   }

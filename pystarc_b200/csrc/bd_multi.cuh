@@ -20,6 +20,7 @@ struct MultiTab {
   long long total;
   unsigned long long* ctr;  // shared counters: pending cursor over global indices, tallies
   int small, large;         // every ligand has at most 32, at least 128 atoms, and no contact forces
+  int largest;              // atoms of the largest ligand
 
   // the interface of the split stepper's kernels (OneTab is the single-system one)
   __device__ __forceinline__ const DevSystem& sys(int k) const { return sys_[k]; }
@@ -28,6 +29,7 @@ struct MultiTab {
   __device__ __forceinline__ int global_id(int k, int id) const { return (int)(base[k] + id); }
   __device__ __forceinline__ bool small_ligands() const { return small; }
   __device__ __forceinline__ bool large_ligands() const { return large; }
+  __device__ __forceinline__ int largest_ligand() const { return largest; }
   __device__ __forceinline__ void refill(Traj& tr, int& k, bool& dead, int lane) const;
   __device__ __forceinline__ bool overlap(int k, const double cn[3], bool need, int lane, const RecView&) const;
 };

@@ -68,6 +68,7 @@ struct OneTab {
   __device__ __forceinline__ bool small_ligands() const { return S.n_lig <= 32 && !S.wca; }
   // ligands worth sharing among warps: every one of at least 128 atoms, no contact forces
   __device__ __forceinline__ bool large_ligands() const { return S.n_lig >= 128 && !S.wca; }
+  __device__ __forceinline__ int largest_ligand() const { return S.n_lig; }  // atoms
   __device__ __forceinline__ void refill(Traj& tr, int&, bool& dead, int lane) const { warp_refill(P, tr, dead, lane); }
   __device__ __forceinline__ bool overlap(int, const double cn[3], bool need, int lane, const RecView& v) const {
     return warp_overlap(S, cn, need, lane, v);
@@ -230,7 +231,7 @@ __global__ void __launch_bounds__(kStepBlock, 4) split_step_kernel(const __grid_
   if (END) stats_block_end(P0, sh.stats);
 }
 
-// The next item of a warp after its first: the cursor counts the items taken beyond one per warp.
+// The next turn of a warp after its first: the cursor counts the turns taken beyond one per warp.
 __device__ __forceinline__ int next_item(int* cursor, int n_warps, int lane) {
   int j = 0;
   if (lane == 0) j = n_warps + atomicAdd(cursor, 1);
@@ -386,12 +387,26 @@ __device__ __forceinline__ int fwd_warps(int n, int n_warps) {
   return n * 8 <= n_warps ? 8 : n * 4 <= n_warps ? 4 : n * 2 <= n_warps ? 2 : 1;
 }
 
+// List entries a warp takes at a time in split_fwd_kernel<LONG>: about eight turns per warp and at most 16
+// entries, or 512 atoms of ligands above 64 (a last turn of long poses would leave other warps waiting).
+// The cursor is one address, and the device adds to it about once a nanosecond: with an entry a turn, lists
+// of 100,000 poses and more were bound by it (256 steps, far-field of 18 atoms, FP64: 300,000 poses
+// 76.7 -> 61.4 ms, 100,000 27.4 -> 23.2; 18 atoms with grids and Born direction 2 160 -> 142; 40 atoms,
+// mixed, 85.8 -> 71.7; 200 atoms, 300,000 246 -> 240, 100,000 level).  Neighbours in the list share the
+// sectors of their poses and forces (a turn's entries far apart: 69 instead of 59 ms at 600,000).
+constexpr int kLongTurns = 8;
+__device__ __forceinline__ int fwd_turn(int n, int n_warps, int atoms) {
+  return n < 2 * kLongTurns * n_warps ? 1
+                                      : max(1, min(n / (kLongTurns * n_warps), atoms <= 64 ? 16 : min(16, 512 / atoms)));
+}
+
 // Forces on the ligand atoms of the listed poses: a warp per pose, or four poses per warp for small
 // ligands in mixed precision and lists of several poses a warp (18 atoms, 150,000 slots: 155 -> 116 us;
 // at 8,000 slots a warp per pose is the faster, 15.5 against 17.4 us, and in FP64 the quarter-warp
 // form spills and is slower at 30,011).  Bound by latency at 13 warps per SM: issue slots 45 %, L1 43 %,
-// the double-float conversions 22 %.
-template <typename FT, bool TORQUE, class TAB>
+// the double-float conversions 22 %.  LONG: several entries a turn, for pools that can list 16 poses per
+// warp; a kernel of its own, because the loop over a turn cost lists with one entry a turn 2 %.
+template <typename FT, bool TORQUE, bool LONG, class TAB>
 __global__ void __launch_bounds__(256, 2) split_fwd_kernel(const __grid_constant__ TAB T, SlotBuf B, SplitBuf U,
                                                            int set) {
   const unsigned FULL = 0xffffffffu;
@@ -448,7 +463,8 @@ __global__ void __launch_bounds__(256, 2) split_fwd_kernel(const __grid_constant
       }
     }
   } else {
-    for (int j = first; j < n; j = next_item(U.cnt + 4 * set + 2, n_warps, lane)) {
+    const int m = LONG ? fwd_turn(n, n_warps, T.largest_ligand()) : 1;
+    for (int j = first * m, left = m; j < n;) {
       const int slot = U.flist[j];
       int id = B.traj[slot];
       const DevSystem& S = T.sys(T.locate(id));
@@ -458,6 +474,11 @@ __global__ void __launch_bounds__(256, 2) split_fwd_kernel(const __grid_constant
                                                              PosFromPose{pose.R, pose.c}, f, t, e, cnt,
                                                              RecView{nullptr, nullptr});
       store_force(U, slot, lane, f, t);
+      if (LONG && --left) ++j;
+      else {
+        j = m * next_item(U.cnt + 4 * set + 2, n_warps, lane);
+        left = m;
+      }
     }
   }
   const unsigned ng = gsumu<32>(cnt.grid, FULL), nf = gsumu<32>(cnt.ff, FULL);

@@ -61,3 +61,17 @@ def _assert_same(s, n, steps, precision, torque, **kw):
 def test_four_small_ligands_share_a_warp(n_of, torque):
     s = dataclasses.replace(system("c2"), r_start=14.0, r_escape=40.0)  # some poses near, some far
     _assert_same(s, n_of(16 * _sms()), 4, "mixed", torque)
+
+
+# a warp takes several entries a turn from 16 poses per warp on: 16 at most, 512 atoms of larger ligands
+@pytest.mark.parametrize("n_of", [lambda w: 16 * w - 1, lambda w: 16 * w, lambda w: 25 * w + 5, lambda w: 130 * w + 7])
+@pytest.mark.parametrize("atoms", [18, 90])
+def test_a_warp_takes_several_poses_a_turn(n_of, atoms):
+    from pystarc_b200 import synth
+
+    if atoms == 18:
+        s = dataclasses.replace(system("c2"), r_start=14.0, r_escape=40.0, lig_born_grids=[])
+    else:
+        s = dataclasses.replace(synth.config3(scale=0.4, device="cuda"), r_start=20.0, r_escape=60.0, lig_born_grids=[])
+    assert len(s.lig_q) >= atoms
+    _assert_same(s, n_of(16 * _sms()), 3, "fp64" if atoms == 18 else "mixed", "centroid")
