@@ -822,11 +822,12 @@ int eval_batch(BdHandle* h, PoseBatch P, int prec, int torque, cudaStream_t s) {
     CK(h, cudaLaunchKernel(t.pose_block, dim3((unsigned)P.n), dim3(256), args, 0, s));
     return BD_OK;
   }
-  const long long want = (P.n + 7) / 8;  // a warp per pose
-  const int b_fwd = (int)std::min<long long>(want, persistent_blocks(h, t.pose_fwd, 256)),
-            b_rev = (int)std::min<long long>(want, persistent_blocks(h, t.pose_rev, 256));
-  CK(h, cudaLaunchKernel(t.pose_fwd, dim3(b_fwd), dim3(256), args, 0, s));
-  if (h->S.born_rev && (h->S.terms & BD_TERM_REV_BORN)) CK(h, cudaLaunchKernel(t.pose_rev, dim3(b_rev), dim3(256), args, 0, s));
+  // light poses stride over resident warps: handing out a block each costs as much as they do (18 atoms, no
+  // sweep, mixed, 100,000 poses 134 us, 140 with a block each)
+  const bool rev = h->S.born_rev && (h->S.terms & BD_TERM_REV_BORN);
+  const int blocks = (int)std::min<long long>(P.n, (long long)h->n_sm * (rev || h->S.n_lig > 96 ? 512 : 16));
+  CK(h, cudaLaunchKernel(t.pose_fwd, dim3(blocks), dim3(32), args, 0, s));
+  if (rev) CK(h, cudaLaunchKernel(t.pose_rev, dim3(blocks), dim3(32), args, 0, s));
   return BD_OK;
 }
 

@@ -3,12 +3,15 @@
 //
 //   pose_block_kernel  one block per pose, for batches that would leave SMs idle otherwise: its
 //                      eight warps share the ligand atoms and then the sweep of Born direction 2
-//   pose_fwd_kernel    forces on the ligand atoms, one warp per pose (four poses per warp for
-//                      small ligands in mixed precision)
+//   pose_fwd_kernel    forces on the ligand atoms, one warp per pose
 //   pose_rev_kernel    Born direction 2, one warp per pose, added to the forces of the former
 //
-// One kernel for both parts held 168 registers a thread (12 warps per SM); apart, the sweep runs
-// at 64 with 32 warps per SM.  Every sum keeps the order of the one-warp evaluation.
+// One kernel for both parts held 168 registers a thread (12 warps per SM); apart, the ligand atoms run at
+// 128 and 16 warps, the sweep at 64 and 32 in mixed precision without torque, at 80 and 24 with torque, at
+// 128 and 16 in FP64.  The last two run in blocks of one warp, handed out by the device: poses differ in
+// cost, and resident blocks of eight warps that stride left the last of their rounds nearly empty (3,200 +
+// 18 atoms, mixed, 8,000 poses 159 -> 99 us, 100,000 820 -> 700).  Every sum keeps the order of the one-warp
+// evaluation.
 #pragma once
 
 #include "bd_split.cuh"
@@ -122,14 +125,12 @@ __global__ void __launch_bounds__(256, 2) pose_block_kernel(const __grid_constan
 }
 
 template <typename FT, bool TORQUE>
-__global__ void __launch_bounds__(256, 2) pose_fwd_kernel(const __grid_constant__ DevSystem S,
+__global__ void __launch_bounds__(32, 16) pose_fwd_kernel(const __grid_constant__ DevSystem S,
                                                           const __grid_constant__ PoseBatch P) {
   const unsigned FULL = 0xffffffffu;
-  const int lane = threadIdx.x & 31;
-  const long long n_warps = ((long long)gridDim.x * blockDim.x) >> 5;
-  const long long first = (threadIdx.x >> 5) * (long long)gridDim.x + blockIdx.x;
+  const int lane = threadIdx.x;
   Counts cnt{0, 0, 0};
-  for (long long t = first; t < P.n; t += n_warps) {
+  for (long long t = blockIdx.x; t < P.n; t += gridDim.x) {
     const Pose<BatchSrc> pose(BatchSrc{P, t});
     double f[3], tq[3], e;
     group_forces<FT, 32, TORQUE, true, BatchPos, false>(
@@ -142,20 +143,19 @@ __global__ void __launch_bounds__(256, 2) pose_fwd_kernel(const __grid_constant_
 }
 
 template <typename FT, bool TORQUE>
-__global__ void __launch_bounds__(256, sizeof(FT) == 4 ? (TORQUE ? 3 : 4) : 2) pose_rev_kernel(const __grid_constant__ DevSystem S,
-                                                                               const __grid_constant__ PoseBatch P) {
+__global__ void __launch_bounds__(32, sizeof(FT) == 4 ? (TORQUE ? 24 : 32) : 16) pose_rev_kernel(
+    const __grid_constant__ DevSystem S, const __grid_constant__ PoseBatch P) {
   using V4 = typename Vec4<FT>::type;
-  __shared__ V4 bufs[8][kSplitBuf<FT>];
+  __shared__ V4 buf[kSplitBuf<FT>];
   const unsigned FULL = 0xffffffffu;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const long long n_warps = ((long long)gridDim.x * blockDim.x) >> 5;
+  const int lane = threadIdx.x;
   unsigned nr = 0;
-  for (long long t = warp * (long long)gridDim.x + blockIdx.x; t < P.n; t += n_warps) {
+  for (long long t = blockIdx.x; t < P.n; t += gridDim.x) {
     const double c[3] = {P.cen[3 * t], P.cen[3 * t + 1], P.cen[3 * t + 2]};
     if (!needs_reverse(S, c)) continue;
     const BatchSrc src{P, t};
     double r[3] = {0, 0, 0}, u[3] = {0, 0, 0};
-    lean_reverse_born<FT, TORQUE, true>(S, src, lane, bufs[warp], r, u, nr);
+    lean_reverse_born<FT, TORQUE, true>(S, src, lane, buf, r, u, nr);
 #pragma unroll
     for (int i = 0; i < 3; ++i) {
       r[i] = gsum<32>(r[i], FULL);
