@@ -797,35 +797,34 @@ size_t stepper_smem(const DevSystem& S, const DevSim& P, void* fn) {
 }
 
 // Forces of a batch of poses.  Groups of 1 to 16 lanes (tiny ligands with nothing to sweep, or the
-// caller's choice) run one kernel; whole warps run the split force code.  A block per pose is the faster
-// up to 24 poses per SM (a warp per pose takes 50-90 us however few there are): protein + small ligand
-// FP64, 37 poses 53 us before -> 21, 592 55 -> 30, 1,500 68 -> 58 (100 with a warp per pose); 3,000 poses
-// by warps 124 -> 135, 20,000 607 -> 389, 100,000 mixed 1,240 -> 920; protein-protein FP64 37 poses
-// 168 -> 42, 6,000 1,119 -> 808.
+// caller's choice) run one kernel; whole warps run one of three forms (eval_form), the same bits in each.
 int eval_batch(BdHandle* h, PoseBatch P, int prec, int torque, cudaStream_t s) {
   const KernelTable& t = table_for(prec, torque);
   const int G = launch_group(h);
+  const bool rev = h->S.born_rev && (h->S.terms & BD_TERM_REV_BORN);
+  int one = 4;  // index of the one-kernel form: whole warps, or smaller groups
   for (int i = 0; i < 4; ++i)
-    if (kGroups[i] == G) {
-      const int block = 128;
-      const long long per_block = block / G;
-      const int blocks = (int)std::min<long long>((P.n + per_block - 1) / per_block, (long long)h->n_sm * 64);
-      unsigned long long* ctr = nullptr;
-      void* pose_args[] = {&h->S, &P.n, &P.cen, &P.rot, &P.rot_is_matrix, &P.F, &P.T, &P.E, &ctr};
-      void* atom_args[] = {&h->S, &P.n, &P.atoms, &P.rot, &P.cen, &P.F, &P.T, &P.E};
-      CK(h, cudaLaunchKernel(P.atoms ? t.atoms[i] : t.pose[i], dim3(blocks), dim3(block),
-                             P.atoms ? atom_args : pose_args, 0, s));
-      return BD_OK;
-    }
+    if (kGroups[i] == G) one = i;
+  const int units = (h->S.n_lig + 31) / 32 + (rev ? h->S.n_chunks : 0);
+  const int form = one < 4 ? EVAL_ONE : eval_form(P.n, h->n_sm, units, prec == BD_PREC_FP64, rev, h->S.wca != 0);
+  if (form == EVAL_ONE) {
+    const int block = 128, per_block = block / kGroups[one];
+    const int blocks = (int)std::min<long long>((P.n + per_block - 1) / per_block, (long long)h->n_sm * 64);
+    unsigned long long* ctr = nullptr;
+    void* pose_args[] = {&h->S, &P.n, &P.cen, &P.rot, &P.rot_is_matrix, &P.F, &P.T, &P.E, &ctr};
+    void* atom_args[] = {&h->S, &P.n, &P.atoms, &P.rot, &P.cen, &P.F, &P.T, &P.E};
+    CK(h, cudaLaunchKernel(P.atoms ? t.atoms[one] : t.pose[one], dim3(blocks), dim3(block),
+                           P.atoms ? atom_args : pose_args, 0, s));
+    return BD_OK;
+  }
   void* args[] = {&h->S, &P};
-  if (P.n <= (long long)kBlockPoses * h->n_sm && !h->S.wca) {
-    CK(h, cudaLaunchKernel(t.pose_block, dim3((unsigned)P.n), dim3(256), args, 0, s));
+  if (form == EVAL_BLOCK) {
+    CK(h, cudaLaunchKernel(h->S.wca ? t.pose_block_contact : t.pose_block, dim3((unsigned)P.n), dim3(256), args, 0, s));
     return BD_OK;
   }
   // light poses stride over resident warps: handing out a block each costs as much as they do (18 atoms, no
-  // sweep, mixed, 100,000 poses 134 us, 140 with a block each)
-  const bool rev = h->S.born_rev && (h->S.terms & BD_TERM_REV_BORN);
-  const int blocks = (int)std::min<long long>(P.n, (long long)h->n_sm * (rev || h->S.n_lig > 96 ? 512 : 16));
+  // sweep, 100,000 poses 134 us, 140 with a block each)
+  const int blocks = (int)std::min<long long>(P.n, (long long)h->n_sm * (rev || units >= 4 ? 512 : 16));
   CK(h, cudaLaunchKernel(t.pose_fwd, dim3(blocks), dim3(32), args, 0, s));
   if (rev) CK(h, cudaLaunchKernel(t.pose_rev, dim3(blocks), dim3(32), args, 0, s));
   return BD_OK;

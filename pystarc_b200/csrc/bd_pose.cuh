@@ -60,9 +60,28 @@ __device__ __forceinline__ bool needs_reverse(const DevSystem& S, const double c
   return (S.terms & 4u) && S.born_rev && norm3(c[0], c[1], c[2]) - S.rec_max_r < S.lig_born_rho;
 }
 
-constexpr int kBlockPoses = 24;  // batches of at most this many poses per SM take a block each
+// Which form evaluates n poses, by the work of one pose that warps can share: units of 32 ligand atoms, or of
+// 32 receptor atoms to sweep.
+//   EVAL_BLOCK  a block per pose: short batches wait for one pose's chain, which eight warps shorten (3,200 +
+//               18 atoms FP64, 37 poses: 55 us in one kernel, 58 by warps, 23 by blocks).  With little to
+//               share a pose keeps one warp of eight busy, and contact forces come from one warp anyway
+//   EVAL_ONE    both parts in one kernel, four warps a block: short batches of light poses, where a second
+//               launch is a quarter of the time (87 + 18 atoms FP64, 600 poses: 13 us, 19 by warps, 21 by
+//               blocks), and medium ones in FP64, whose registers the 128 of the other forms do not hold
+//   EVAL_WARPS  a kernel for the ligand atoms and one for the sweep, a warp per pose
+// The lines, us by blocks / by warps: 3,200 + 18 atoms FP64 1,500 poses 60 / 67, 2,000 75 / 71; 1,701 + 1,401
+// mixed 1,184 177 / 189, 1,500 216 / 198; FP64 without a sweep 3,000 259 / 312; 213 + 176 FP64 600 28 / 36,
+// 1,000 40 / 40 and 29 in one; contact forces, 213 + 176 FP64, 37 poses 443 / 460 and 426 in one.
+enum { EVAL_ONE, EVAL_BLOCK, EVAL_WARPS };
+inline int eval_form(long long n, int n_sm, int units, bool fp64, bool rev, bool wca) {
+  const int block = units >= 32 ? (fp64 && !rev ? 24 : 12) : units >= 6 && !wca ? 6 : 0;  // poses per SM
+  const int one = fp64 && units < 32 ? 9 : units < 8 ? (rev ? 20 : 6) : 0;
+  return n <= (long long)block * n_sm ? EVAL_BLOCK : n <= (long long)one * n_sm ? EVAL_ONE : EVAL_WARPS;
+}
 
-template <typename FT, bool TORQUE>
+// CONTACT: systems with contact forces.  One warp adds them to the lanes' sums, atom by atom as in the
+// one-warp evaluation, while the others wait; a kernel of its own, so that systems without keep theirs.
+template <typename FT, bool TORQUE, bool CONTACT>
 __global__ void __launch_bounds__(256, 2) pose_block_kernel(const __grid_constant__ DevSystem S,
                                                             const __grid_constant__ PoseBatch P) {
   using V4 = typename Vec4<FT>::type;
@@ -75,6 +94,7 @@ __global__ void __launch_bounds__(256, 2) pose_block_kernel(const __grid_constan
   };
   __shared__ Shared sh;
   __shared__ double out[16];
+  __shared__ double sums[CONTACT ? (TORQUE ? 6 : 3) : 1][32];
   __shared__ int cnts[16];
   const unsigned FULL = 0xffffffffu;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -83,8 +103,31 @@ __global__ void __launch_bounds__(256, 2) pose_block_kernel(const __grid_constan
     const BatchSrc src{P, t};
     const Pose<BatchSrc> pose(src);
     double tot[4];
-    group_forward<FT, TORQUE, true>(S, BatchPos{pose.R, pose.c, P.atoms ? P.atoms + t * S.n_lig * 3 : nullptr}, lane,
-                                    warp, 8, 1, sh.fwd, S.terms & 1u, S.terms & 2u, tot, cnt);
+    const BatchPos pos{pose.R, pose.c, P.atoms ? P.atoms + t * S.n_lig * 3 : nullptr};
+    auto contact = [&](double* tot) {
+      if constexpr (CONTACT) {
+        if (!(S.terms & 8u) || !(norm3(pose.c[0], pose.c[1], pose.c[2]) < S.wca_act)) return;
+        constexpr int N = TORQUE ? 6 : 3;
+        if (warp < N) sums[warp][lane] = tot[0];
+        __syncthreads();
+        if (warp == 0) {
+          double f[3] = {sums[0][lane], sums[1][lane], sums[2][lane]}, u[3] = {0, 0, 0};
+          if (TORQUE) {
+#pragma unroll
+            for (int i = 0; i < 3; ++i) u[i] = sums[N - 3 + i][lane];
+          }
+          group_contact<32, TORQUE>(S, pose.c, lane, FULL, pos, f, u);
+#pragma unroll
+          for (int i = 0; i < 3; ++i) {
+            sums[i][lane] = f[i];
+            if (TORQUE) sums[N - 3 + i][lane] = u[i];
+          }
+        }
+        __syncthreads();
+        if (warp < N) tot[0] = sums[warp][lane];
+      }
+    };
+    group_forward<FT, TORQUE, true>(S, pos, lane, warp, 8, 1, sh.fwd, S.terms & 1u, S.terms & 2u, tot, cnt, contact);
     if (lane == 0 && warp < NC) out[warp] = tot[0];
     const bool rev = needs_reverse(S, pose.c);
     double r[3] = {0, 0, 0}, u[3] = {0, 0, 0};

@@ -327,13 +327,18 @@ __device__ __forceinline__ void group_sync(int id, int threads) {
 // W rows of NC components of 32 lanes); component k is then summed by warp k mod W, lane by lane in the
 // order of the atoms, as a single warp sums them: the same bits.  tot[i] receives component gw + i * W
 // (f0..f2, t0..t2 with TORQUE, the energy last with ENERGY), reduced over the lanes.  Contact forces are
-// not included.
+// not included; `extra`, called by every warp with its lane's sums, may add them.
 template <bool TORQUE, bool ENERGY>
 constexpr int kForwardNc = 3 + (TORQUE ? 3 : 0) + (ENERGY ? 1 : 0);
 
-template <typename FT, bool TORQUE, bool ENERGY, class PosFn>
+struct NoExtra {
+  __device__ __forceinline__ void operator()(double*) const {}
+};
+
+template <typename FT, bool TORQUE, bool ENERGY, class PosFn, class Extra = NoExtra>
 __device__ __forceinline__ void group_forward(const DevSystem& S, const PosFn& pos, int lane, int gw, int W, int bar,
-                                              double* sh, bool t_grid, bool t_ff, double tot[4], Counts& cnt) {
+                                              double* sh, bool t_grid, bool t_ff, double tot[4], Counts& cnt,
+                                              const Extra& extra = Extra{}) {
   constexpr int NC = kForwardNc<TORQUE, ENERGY>;
 #pragma unroll
   for (int i = 0; i < 4; ++i) tot[i] = 0.0;
@@ -373,6 +378,7 @@ __device__ __forceinline__ void group_forward(const DevSystem& S, const PosFn& p
     }
     flip ^= 1;
   }
+  extra(tot);
 #pragma unroll
   for (int k = 0; k < 4; ++k)
     if (gw + k * W < NC) tot[k] = gsum<32>(tot[k], 0xffffffffu);

@@ -11,7 +11,7 @@
 
 namespace bd {
 
-constexpr int kGroups[5] = {1, 4, 8, 16, 32};  // lanes per trajectory of step_kernel and (up to 16) eval_*_kernel
+constexpr int kGroups[5] = {1, 4, 8, 16, 32};  // lanes per trajectory of step_kernel and eval_*_kernel
 
 struct SplitKernels {
   void *first, *mid, *last;  // scalar kernel: begin, end + begin, end
@@ -19,8 +19,8 @@ struct SplitKernels {
 };
 
 struct KernelTable {
-  void *pose[4], *atoms[4], *step[5];  // by kGroups
-  void *pose_block, *pose_fwd, *pose_rev;  // evaluation by whole warps
+  void *pose[5], *atoms[5], *step[5];  // by kGroups
+  void *pose_block, *pose_block_contact, *pose_fwd, *pose_rev;  // evaluation by whole warps
   void *warp, *warp_capped;            // step_kernel_warp without a register cap and at 128
   void *sur_begin, *sur_end;
   SplitKernels split, multi;           // of one system, of a heterogeneous batch
@@ -36,12 +36,14 @@ SplitKernels split_kernels() {
 template <typename FT, bool TQ>
 KernelTable make_table() {
   return {{(void*)&eval_pose_kernel<FT, 1, TQ>, (void*)&eval_pose_kernel<FT, 4, TQ>, (void*)&eval_pose_kernel<FT, 8, TQ>,
-           (void*)&eval_pose_kernel<FT, 16, TQ>},
+           (void*)&eval_pose_kernel<FT, 16, TQ>, (void*)&eval_pose_kernel<FT, 32, TQ>},
           {(void*)&eval_atoms_kernel<FT, 1, TQ>, (void*)&eval_atoms_kernel<FT, 4, TQ>,
-           (void*)&eval_atoms_kernel<FT, 8, TQ>, (void*)&eval_atoms_kernel<FT, 16, TQ>},
+           (void*)&eval_atoms_kernel<FT, 8, TQ>, (void*)&eval_atoms_kernel<FT, 16, TQ>,
+           (void*)&eval_atoms_kernel<FT, 32, TQ>},
           {(void*)&step_kernel<FT, 1, TQ>, (void*)&step_kernel<FT, 4, TQ>, (void*)&step_kernel<FT, 8, TQ>,
            (void*)&step_kernel<FT, 16, TQ>, (void*)&step_kernel<FT, 32, TQ>},
-          (void*)&pose_block_kernel<FT, TQ>,
+          (void*)&pose_block_kernel<FT, TQ, false>,
+          (void*)&pose_block_kernel<FT, TQ, true>,
           (void*)&pose_fwd_kernel<FT, TQ>,
           (void*)&pose_rev_kernel<FT, TQ>,
           (void*)&step_kernel_warp<FT, TQ, 1>,
