@@ -34,7 +34,8 @@ constexpr int kStepBlock = 128;  // threads of a scalar-kernel block
 struct SplitBuf {
   double* F;       // 3 * cap: forces on the ligand atoms; the step's total force once complete
   double* T;       // 3 * cap
-  double* rv;      // 6 * cap: Born direction 2 sums r (ligand frame) and u, from the sweep
+  double* rv;      // 6 * cap: Born direction 2 sums r (ligand frame) and u, from the sweep (64-bit indexes:
+                   // the pose arrays allow 2^29 slots)
   double* rprev;   // cap: |c| at the end of the previous step (statistics)
   int8_t* mode;    // 0: no step; 1: F, T to be used as they are; 2: reused (complete);
                    // 3: F, T plus the Born direction 2 sums in rv
@@ -131,8 +132,8 @@ __global__ void __launch_bounds__(kStepBlock, 4) split_step_kernel(const __grid_
         for (int i = 0; i < 3; ++i) {
           F[i] = U.F[3 * slot + i];
           Tq[i] = U.T[3 * slot + i];
-          rv[i] = U.rv[6 * slot + i];
-          rv[3 + i] = U.rv[6 * slot + 3 + i];
+          rv[i] = U.rv[6 * (size_t)slot + i];
+          rv[3 + i] = U.rv[6 * (size_t)slot + 3 + i];
         }
       }
       const bool need = mode != 0;
@@ -390,7 +391,7 @@ __device__ __forceinline__ void group_forward(const DevSystem& S, const PosFn& p
 // warp per pose -> with this rule: 100 trajectories 15.7 -> 6.5 ms, 700 18.1 -> 10.8, 2,000 22.8 -> 21.9,
 // 6,000 34.9 both (two or eight warps there: 10 % slower, the rounds' barriers).
 __device__ __forceinline__ int fwd_warps(int n, int n_warps) {
-  return n * 8 <= n_warps ? 8 : n * 4 <= n_warps ? 4 : n * 2 <= n_warps ? 2 : 1;
+  return n <= n_warps / 8 ? 8 : n <= n_warps / 4 ? 4 : n <= n_warps / 2 ? 2 : 1;
 }
 
 // List entries a warp takes at a time in split_fwd_kernel<LONG>: about eight turns per warp and at most 16
@@ -811,7 +812,7 @@ __device__ __forceinline__ void group_reverse_born(const DevSystem& S, const SRC
 // from 120 to 40 ms with eight; 8,000 mixed 200 -> 136 ms, 30,011 FP64 170 -> 147 ms.  Lines twice
 // and four times as far out are no better (8,000: 142 and 134 ms; 30,011 FP64: 172 and 168 ms).
 __device__ __forceinline__ int rev_warps(int n, int n_warps) {
-  return n * 4 <= n_warps ? 8 : n * 2 <= n_warps ? 4 : n <= n_warps ? 2 : 1;
+  return n <= n_warps / 4 ? 8 : n <= n_warps / 2 ? 4 : n <= n_warps ? 2 : 1;
 }
 
 // FP32 without torque: capped at 64 registers, 32 warps per SM (at 80 and 24 warps 150,000 trajectories
@@ -849,14 +850,14 @@ __global__ void __launch_bounds__(256, sizeof(FT) == 4 ? (TORQUE ? 3 : 4) : 2) s
       r[0] = gsum<32>(r[0], FULL);
       r[1] = gsum<32>(r[1], FULL);
       r[2] = gsum<32>(r[2], FULL);
-      if (lane < 3) U.rv[6 * slot + lane] = r[lane];
-      if (!TORQUE && lane < 3) U.rv[6 * slot + 3 + lane] = 0.0;
+      if (lane < 3) U.rv[6 * (size_t)slot + lane] = r[lane];
+      if (!TORQUE && lane < 3) U.rv[6 * (size_t)slot + 3 + lane] = 0.0;
     }
     if (TORQUE && gw == (W > 1 ? 1 : 0)) {
       u[0] = gsum<32>(u[0], FULL);
       u[1] = gsum<32>(u[1], FULL);
       u[2] = gsum<32>(u[2], FULL);
-      if (lane < 3) U.rv[6 * slot + 3 + lane] = u[lane];
+      if (lane < 3) U.rv[6 * (size_t)slot + 3 + lane] = u[lane];
     }
   }
   nr = gsumu<32>(nr, FULL);
