@@ -86,7 +86,7 @@ struct BdHandle {
   // split stepper (BD_GROUP_SPLIT): per-slot scratch of one step
   SplitBuf split_buf{};
   int split_cap = 0;
-  cudaStream_t side = nullptr;  // the force kernel that runs beside the other (captured, or a first launch)
+  cudaStream_t side = nullptr;  // capture only: the force kernel that runs beside the other
   cudaEvent_t fork = nullptr, join = nullptr;
   unsigned long long* sur_ctr_host_base = nullptr;
   // graphs, one per slot buffer, and the bytes of everything that was captured into them
@@ -1450,7 +1450,7 @@ struct SplitPlan {
   bool rev;        // some system has Born direction 2
   size_t smem;     // of the scalar kernel when it ends a step
   int b_step, b_fwd, b_rev;
-  cudaStream_t side;
+  cudaStream_t side;  // capture only, else null: the two then follow one another
   cudaEvent_t fork, join;
   unsigned long long* ctr;
   int n_sm;
@@ -1468,14 +1468,16 @@ cudaError_t enqueue_split_steps(const SplitPlan& p, SlotBuf src, SlotBuf dst, co
     if (!ok(cudaLaunchKernel(fn, dim3(p.b_step), dim3(kStepBlock), s_args, k == 0 ? 0 : p.smem, s))) return e;
     if (k == K) break;
     void* f_args[] = {p.tab, &src, &U, &set};
-    if (p.rev) {
+    if (p.rev && !p.side) {
+      if (!ok(cudaLaunchKernel(p.kn->rev, dim3(p.b_rev), dim3(256), f_args, 0, s))) return e;
+    } else if (p.rev) {
       if (!ok(cudaEventRecord(p.fork, s)) || !ok(cudaStreamWaitEvent(p.side, p.fork, 0)) ||
           !ok(cudaLaunchKernel(p.kn->rev, dim3(p.b_rev), dim3(256), f_args, 0, p.side)) ||
           !ok(cudaEventRecord(p.join, p.side)))
         return e;
     }
     if (!ok(cudaLaunchKernel(p.fwd, dim3(p.b_fwd), dim3(256), f_args, 0, s))) return e;
-    if (p.rev && !ok(cudaStreamWaitEvent(s, p.join, 0))) return e;
+    if (p.rev && p.side && !ok(cudaStreamWaitEvent(s, p.join, 0))) return e;
   }
   compact_kernel<<<p.n_sm * 4, 256, 0, s>>>(src, dst, live, p.ctr);
   if (!ok(cudaGetLastError())) return e;
@@ -1487,8 +1489,9 @@ cudaError_t enqueue_split_steps(const SplitPlan& p, SlotBuf src, SlotBuf dst, co
 // instantiating 64 split steps takes 3-5 ms a graph, so where neither graph exists the first launch goes to
 // the stream as it is (`direct`) and each graph is built behind the launches before it: four systems of 20 to
 // 124 atoms in a batch, 100,000 trajectories, 64 steps: 20.4 -> 13.4 ms (14.1 with one fused launch; mixed
-// 19.1 -> 11.9, fused 12.3).  On a stream that is being captured
-// the graphs come first, so that none of its work is left on the side stream.
+// 19.1 -> 11.9, fused 12.3).  The direct launch stays on its one stream: once a second stream has run
+// kernels, every step of every graph takes 0.4-0.7 us more (1,000 slots, 512 steps: 12.8 -> 13.1 ms).  A
+// stream that is being captured gets the graphs first.
 extern "C++" {
 template <class Direct, class Build, class Check>
 int run_launches(cudaGraphExec_t* graph, int& cur, int n_launch, bool split, cudaStream_t s, Direct direct,
@@ -1521,7 +1524,7 @@ void* split_fwd(const SplitKernels& kn, int cap, int warps, int precision, bool 
   return cap >= 2 * kLongTurns * warps && !(precision == BD_PREC_MIXED && small) ? kn.fwd_long : kn.fwd;
 }
 
-int enqueue_split_launch(BdHandle* h, int K, cudaStream_t s, int cur) {
+int enqueue_split_launch(BdHandle* h, int K, cudaStream_t s, int cur, bool capture) {
   const SplitKernels& kn = table_for(h->sp.precision, h->sp.torque_mode).split;
   OneTab T{h->S, h->P};
   SplitPlan p{&kn, kn.fwd, &T, h->split_buf, h->S.born_rev != 0, stepper_smem(h->S, h->P, kn.mid)};
@@ -1530,7 +1533,7 @@ int enqueue_split_launch(BdHandle* h, int K, cudaStream_t s, int cur) {
   p.b_fwd = persistent_blocks(h, kn.fwd, 256);
   p.fwd = split_fwd(kn, h->buf[0].cap, 8 * p.b_fwd, h->sp.precision, h->S.n_lig <= 32 && !h->S.wca);
   p.b_rev = persistent_blocks(h, kn.rev, 256);
-  p.side = h->side;
+  p.side = capture ? h->side : nullptr;
   p.fork = h->fork;
   p.join = h->join;
   p.ctr = h->d_ctr;
@@ -1582,7 +1585,7 @@ int build_graph(BdHandle* h, int K, int c) {
   cudaGraph_t graph;
   CK(h, cudaStreamBeginCapture(h->own, cudaStreamCaptureModeThreadLocal));
   int rc = h->sur ? enqueue_surrogate_launch(h, K, h->own, c, sblocks)
-           : split ? enqueue_split_launch(h, K, h->own, c)
+           : split ? enqueue_split_launch(h, K, h->own, c, true)
                    : enqueue_launch(h, K, h->own, c, fn, smem, blocks);
   cudaError_t e = cudaStreamEndCapture(h->own, &graph);
   if (rc) return rc;
@@ -1606,7 +1609,7 @@ int bd_sim_run(BdHandle* h, int n_launch, int K, void* stream) {
   if (rc) return rc;
   return run_launches(
       h->graph, h->cur, n_launch, !h->sur && launch_group(h) == BD_GROUP_SPLIT, pick(h, stream),
-      [&](cudaStream_t s, int c) { return enqueue_split_launch(h, K, s, c); },
+      [&](cudaStream_t s, int c) { return enqueue_split_launch(h, K, s, c, false); },
       [&](int c) { return build_graph(h, K, c); },
       [&](cudaError_t e) {
         CK(h, e);
@@ -1993,7 +1996,7 @@ int malloc_multi(BdMulti* m, void** p, size_t bytes) {
 }
 
 // K split steps of the pool on buffer c.
-int enqueue_multi_launch(BdMulti* m, int K, cudaStream_t s, int c) {
+int enqueue_multi_launch(BdMulti* m, int K, cudaStream_t s, int c, bool capture) {
   const SplitKernels& kn = table_for(m->precision, m->torque).multi;
   auto blocks = [&](void* fn, int block) {
     int per_sm = 0;
@@ -2006,7 +2009,7 @@ int enqueue_multi_launch(BdMulti* m, int K, cudaStream_t s, int c) {
   p.b_fwd = blocks(kn.fwd, 256);
   p.fwd = split_fwd(kn, m->cap, 8 * p.b_fwd, m->precision, m->T.small);
   p.b_rev = blocks(kn.rev, 256);
-  p.side = m->side;
+  p.side = capture ? m->side : nullptr;
   p.fork = m->fork;
   p.join = m->join;
   p.ctr = m->T.ctr;
@@ -2019,7 +2022,7 @@ int multi_graph(BdMulti* m, int K, int c) {
   if (m->graph[c]) return BD_OK;
   cudaGraph_t graph;
   MCK(m, cudaStreamBeginCapture(m->own, cudaStreamCaptureModeThreadLocal));
-  const int rc = enqueue_multi_launch(m, K, m->own, c);
+  const int rc = enqueue_multi_launch(m, K, m->own, c, true);
   cudaError_t e = cudaStreamEndCapture(m->own, &graph);
   if (rc) return rc;
   MCK(m, e);
@@ -2193,7 +2196,7 @@ int bd_multi_run(BdMulti* m, int n_launch, int K, void* stream) {
   }
   return run_launches(
       m->graph, m->cur, n_launch, true, (cudaStream_t)stream,
-      [&](cudaStream_t s, int c) { return enqueue_multi_launch(m, K, s, c); },
+      [&](cudaStream_t s, int c) { return enqueue_multi_launch(m, K, s, c, false); },
       [&](int c) { return multi_graph(m, K, c); },
       [&](cudaError_t e) {
         MCK(m, e);
