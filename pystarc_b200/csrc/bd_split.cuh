@@ -421,17 +421,21 @@ __global__ void __launch_bounds__(256, 2) split_fwd_kernel(const __grid_constant
   const int n = U.cnt[4 * set], n_warps = (gridDim.x * blockDim.x) >> 5;
   const int first = (threadIdx.x >> 5) * gridDim.x + blockIdx.x;
   Counts cnt{0, 0, 0};
-  if (sizeof(FT) == 4 && T.small_ligands() && n > 4 * n_warps) {
+  // Entries of the list that go four to a warp.  With torque the one to three after them take a warp each, one
+  // that has few of the others; without, the lanes past the end repeat a pose, uncounted (with the counts apart
+  // the torque kernel spills 40 bytes more: 150,000 slots +1 %; the tail in the loop below costs the other 1 %).
+  const int packed = sizeof(FT) == 4 && !LONG && T.small_ligands() && n > 4 * n_warps ? (TORQUE ? n & ~3 : n) : 0;
+  if (packed) {
     // lanes read the poses of `m` list entries together, then hand them out four at a time
-    const int m = min(32, 4 * ((n + 4 * n_warps - 1) / (4 * n_warps)));
-    for (long long base = (long long)first * m; base < n; base += (long long)n_warps * m) {
+    const int m = min(32, 4 * ((packed + 4 * n_warps - 1) / (4 * n_warps)));
+    for (long long base = (long long)first * m; base < packed; base += (long long)n_warps * m) {
       const int j = (int)base + lane;
-      const bool have = lane < m && j < n;
+      const bool have = lane < m && j < packed;
       const int slot = have ? U.flist[j] : U.flist[(int)base];
       const Pose<SlotSrc> pose(SlotSrc{B, slot});
       int id = B.traj[slot];
       const int sys = T.locate(id);
-      for (int p = 0; p < m && base + p < n; p += 4) {
+      for (int p = 0; p < m && base + p < packed; p += 4) {
         const int src = p + (lane >> 3);
         double c[3], R[9], f[3], t[3];
 #pragma unroll
@@ -440,16 +444,22 @@ __global__ void __launch_bounds__(256, 2) split_fwd_kernel(const __grid_constant
         for (int i = 0; i < 9; ++i) R[i] = __shfl_sync(FULL, pose.R[i], src);
         const int to = __shfl_sync(FULL, slot, src);
         const DevSystem& S = T.sys(__shfl_sync(FULL, sys, src));
-        Counts mine{0, 0, 0};
-        quarter_forces<FT, TORQUE>(S, c, R, lane & 7, f, t, mine);
-        // past the end of the list the lanes repeat a pose, for the shuffles' sake
-        if (base + src < n) {
+        if (TORQUE) {
+          quarter_forces<FT, TORQUE>(S, c, R, lane & 7, f, t, cnt);
           store_force(U, to, lane & 7, f, t);
-          cnt.grid += mine.grid;
-          cnt.ff += mine.ff;
+        } else {
+          Counts mine{0, 0, 0};
+          quarter_forces<FT, TORQUE>(S, c, R, lane & 7, f, t, mine);
+          if (base + src < n) {
+            store_force(U, to, lane & 7, f, t);
+            cnt.grid += mine.grid;
+            cnt.ff += mine.ff;
+          }
         }
       }
     }
+  }
+  if (packed && !TORQUE) {
   } else if (const int W = T.large_ligands() ? fwd_warps(n, n_warps) : 1; W > 1) {
     constexpr int NC = kForwardNc<TORQUE, false>;
     __shared__ double sh[2 * 8 * NC * 32];
@@ -471,7 +481,7 @@ __global__ void __launch_bounds__(256, 2) split_fwd_kernel(const __grid_constant
     }
   } else {
     const int m = LONG ? fwd_turn(n, n_warps, T.largest_ligand()) : 1;
-    for (int j = first * m, left = m; j < n;) {
+    for (int j = TORQUE && packed ? packed + n_warps - 1 - first : first * m, left = m; j < n;) {
       const int slot = U.flist[j];
       int id = B.traj[slot];
       const DevSystem& S = T.sys(T.locate(id));
@@ -482,6 +492,7 @@ __global__ void __launch_bounds__(256, 2) split_fwd_kernel(const __grid_constant
                                                              RecView{nullptr, nullptr});
       store_force(U, slot, lane, f, t);
       if (LONG && --left) ++j;
+      else if (TORQUE && packed) break;
       else {
         j = m * next_item(U.cnt + 4 * set + 2, n_warps, lane);
         left = m;
