@@ -86,6 +86,7 @@ struct BdHandle {
   // split stepper (BD_GROUP_SPLIT): per-slot scratch of one step
   SplitBuf split_buf{};
   int split_cap = 0;
+  bool fused = false;  // its scratch does not fit the device: the fused step runs the configured pool
   cudaStream_t side = nullptr;  // capture only: the force kernel that runs beside the other
   cudaEvent_t fork = nullptr, join = nullptr;
   unsigned long long* sur_ctr_host_base = nullptr;
@@ -758,7 +759,7 @@ int launch_group_for(const BdHandle* h, int overlap) {
   // reverse Born 127 -> 359 M, 600,000 with it 275 -> 365 M; FP64 150,000 171 -> 265 M, 600,000
   // 209 -> 276 M; protein-protein FP64 6,000 slots 2.8 -> 19.9 M, 60,000 22.8 -> 37.8 M.  At
   // 300,000 slots, mixed, without reverse Born they are level (882 and 879 M).
-  return g == BD_GROUP_WARP ? (int)BD_GROUP_SPLIT : g;
+  return g != BD_GROUP_WARP ? g : h->fused ? (int)BD_GROUP_WARP_CAPPED : (int)BD_GROUP_SPLIT;
 }
 
 int launch_group(const BdHandle* h) { return launch_group_for(h, h->sp.overlap); }
@@ -1148,7 +1149,7 @@ int bd_get_launch(BdHandle* h, int* group, int* block, int* grid) {
 }
 
 namespace {
-int ensure_split_buffers(BdHandle* h);
+int split_or_fused(BdHandle* h);
 }
 
 int bd_sim_configure(BdHandle* h, const BdSimParams* p) {
@@ -1177,6 +1178,7 @@ int bd_sim_configure(BdHandle* h, const BdSimParams* p) {
   h->sur_buf = SurBuf{};
   h->split_cap = 0;
   h->split_buf = SplitBuf{};
+  h->fused = false;
   h->sp = *p;
   // live-slot capacity
   const int G = launch_group(h);
@@ -1270,7 +1272,7 @@ int bd_sim_configure(BdHandle* h, const BdSimParams* p) {
     }
   }
   if (!h->sur && G == BD_GROUP_SPLIT)
-    if ((rc = ensure_split_buffers(h))) return rc;
+    if ((rc = split_or_fused(h))) return rc;
   free_unused(h);
   h->sim_ready = true;
   return BD_OK;
@@ -1430,6 +1432,7 @@ int ensure_split_buffers(BdHandle* h) {
   const int C = h->buf[0].cap;
   if (h->split_cap == C) return BD_OK;
   SplitBuf& U = h->split_buf;
+  U = SplitBuf{};
   if (int rc = split_buffers(U, (size_t)C, [&](void** q, size_t b) { return sim_alloc(h, q, b); })) return rc;
   CK(h, cudaMemset(U.cnt, 0, 8 * sizeof(int)));
   CK(h, cudaDeviceSynchronize());  // the legacy stream's memset, before any stream's launches
@@ -1437,6 +1440,22 @@ int ensure_split_buffers(BdHandle* h) {
   if (!h->fork) CK(h, cudaEventCreateWithFlags(&h->fork, cudaEventDisableTiming));
   if (!h->join) CK(h, cudaEventCreateWithFlags(&h->join, cudaEventDisableTiming));
   h->split_cap = C;
+  return BD_OK;
+}
+
+// The split step's buffers; where they do not fit and the step was not asked for, the fused step, which needs
+// none (the scratch is four fifths of the slots' own memory).
+int split_or_fused(BdHandle* h) {
+  const int rc = ensure_split_buffers(h);
+  if (rc != BD_ERR_OOM || h->launch_user) return rc;
+  cudaGetLastError();
+  SplitBuf& U = h->split_buf;
+  for (void* p : {(void*)U.F, (void*)U.T, (void*)U.rv, (void*)U.rprev, (void*)U.mode, (void*)U.flist, (void*)U.rlist})
+    for (auto& b : h->sim_blocks)
+      if (p && b.p == p) b.used = false;
+  free_unused(h);
+  U = SplitBuf{};
+  h->fused = true;
   return BD_OK;
 }
 
@@ -1546,9 +1565,9 @@ int enqueue_split_launch(BdHandle* h, int K, cudaStream_t s, int cur, bool captu
 // for byte.  The surrogate's step also depends on the ensemble's own buffers and is captured for every
 // configuration.  Drops graphs that are not good for K steps of the configured run.
 int match_graphs(BdHandle* h, int K) {
+  if (!h->sur && launch_group(h) == BD_GROUP_SPLIT)
+    if (int rc = split_or_fused(h)) return rc;
   const int G = launch_group(h);
-  if (!h->sur && G == BD_GROUP_SPLIT)
-    if (int rc = ensure_split_buffers(h)) return rc;
   std::vector<unsigned char> key;
   auto add = [&](const void* v, size_t n) {
     key.insert(key.end(), (const unsigned char*)v, (const unsigned char*)v + n);
