@@ -82,7 +82,7 @@ def autotune(sim, candidates=DEFAULT_CANDIDATES, K=16, launches=4, layouts=(None
 
 
 def autotune_multi(batch, layouts=DEFAULT_LAYOUTS, K=16, launches=4):
-    """Heterogeneous batch: time short bursts of the shared persistent launch with each layout applied
+    """Heterogeneous batch: time short bursts of the shared pool's launches with each layout applied
     to every system, keep the fastest; returns (best layout, {layout: steps/s})."""
     import torch
 

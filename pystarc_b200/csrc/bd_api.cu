@@ -754,11 +754,12 @@ int launch_group_for(const BdHandle* h, int overlap) {
   if (h->launch_user) return h->group;
   const bool sweeps = h->S.born_rev || (overlap && !h->rec.empty());
   const int g = default_group(n_charged(h), sweeps);
-  // the split step is the faster one at every pool size measured (BD steps/s, fused kernel at 128
-  // registers -> split; protein + small ligand from the b-sphere): mixed 8,000 slots without
-  // reverse Born 127 -> 359 M, 600,000 with it 275 -> 365 M; FP64 150,000 171 -> 265 M, 600,000
-  // 209 -> 276 M; protein-protein FP64 6,000 slots 2.8 -> 19.9 M, 60,000 22.8 -> 37.8 M.  At
-  // 300,000 slots, mixed, without reverse Born they are level (882 and 879 M).
+  // The split step is the faster one at nearly every pool measured (GPU ms, fused kernel at 128 registers ->
+  // split; 128 steps from the b-sphere without reverse Born): far field of 18 atoms FP64, 3,000 slots 5.3 ->
+  // 1.7, 100,000 15.1 -> 11.2, 600,000 67.5 -> 59.8; mixed 4.9 -> 1.6, 10.8 -> 7.0, 48.8 -> 30.7; with grids
+  // 600,000 FP64 116 -> 84, mixed 82.6 -> 59.8; contact forces mixed 300,000 48.8 -> 45.4; with reverse Born
+  // FP64 300,000 112 -> 56; 1,401 atoms FP64 3,000 105 -> 9.3, 200,000 171 -> 130.  Level: the far field of
+  // 40 atoms, mixed, from 200,000 slots (600,000 70.1 and 70.7).
   return g != BD_GROUP_WARP ? g : h->fused ? (int)BD_GROUP_WARP_CAPPED : (int)BD_GROUP_SPLIT;
 }
 
@@ -771,9 +772,9 @@ int persistent_blocks(BdHandle* h, void* fn, int block, size_t smem = 0) {
 }
 
 // Resident blocks of h->block threads of a stepper: what the slot pool's size follows from.  The
-// split stepper's kernels have block sizes of their own; its pool stays that of a 128-register
-// kernel of h->block threads (with the shared memory of the fused kernel that was the default for
-// FP64 and without reverse Born), so that saved pools keep their capacity.
+// split stepper's kernels have block sizes of their own; its pool is that of a 128-register kernel of
+// h->block threads with the shared memory of the fused kernel (which runs it where its scratch does not
+// fit), so both steps have pools of one size.  A checkpoint of another size is resumed with its own.
 int resident_blocks(BdHandle* h, int G, void* fn, size_t smem) {
   if (G != BD_GROUP_SPLIT) return persistent_blocks(h, fn, h->block, smem);
   int per_sm = 65536 / 128 / h->block, sm_bytes = 0;

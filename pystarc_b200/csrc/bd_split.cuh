@@ -13,7 +13,8 @@
 // own 32 trajectories one after another, and a pool of 8,000 kept 250 warps busy on 148 SMs
 // (protein + small ligand, 8,000 slots: 74 us of forces in that kernel; 6,000 slots of a
 // 1,401-atom ligand: 1,140 us).  Each kernel also gets the registers that suit it: the scalar
-// step and the forward stencils 128, the latency-bound sweep of direction 2 64 (twice the warps).
+// step and the forward stencils 128, the latency-bound sweep of direction 2 64 in mixed precision (twice
+// the warps), 80 with torque, 128 in FP64.
 // Candidates of the sweep (receptor atoms inside the ligand's Born box, in the ligand frame) go
 // to a per-warp buffer in shared memory and are drained in whole groups of 32, entry i by lane i
 // mod 32, in the order of the fused kernel's ring: every lane sums the same terms in the same
