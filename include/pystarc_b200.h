@@ -222,7 +222,8 @@ int bd_sim_restore(BdHandle* h, const double* c, const double* q, const int32_t*
  * registers capped at 128 per thread), or BD_GROUP_SPLIT (each BD step as three kernels: the
  * scalar part, which lists the poses that need forces, the ligand-atom forces and Born direction 2
  * of the listed poses; the same trajectories as BD_GROUP_WARP; the default wherever there is a
- * receptor to sweep), and threads per block (multiple of 32, <= 256; the split step's kernels have
+ * receptor to sweep and its 113 bytes a slot fit the device, else BD_GROUP_WARP_CAPPED), and threads
+ * per block (multiple of 32, <= 256; the split step's kernels have
  * their own).  Set by the autotuner; 0 keeps the current value. */
 enum { BD_GROUP_WARP = 64, BD_GROUP_WARP_CAPPED = 65, BD_GROUP_SPLIT = 66 };
 int bd_set_launch(BdHandle* h, int group, int block_threads);
