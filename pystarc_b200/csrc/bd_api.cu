@@ -1464,7 +1464,7 @@ int split_or_fused(BdHandle* h) {
 // step do not depend on each other: the sweep is captured on a branch of its own.
 struct SplitPlan {
   const SplitKernels* kn;
-  void* fwd;       // kn->fwd or kn->fwd_long (split_fwd)
+  void* fwd;       // the ligand-atom kernel (split_fwd)
   void* tab;       // OneTab or MultiTab (copied at capture)
   SplitBuf U;
   bool rev;        // some system has Born direction 2
@@ -1538,10 +1538,10 @@ int run_launches(cudaGraphExec_t* graph, int& cur, int n_launch, bool split, cud
 }
 }  // extern "C++"
 
-// The ligand-atom kernel of a pool of `cap` slots: the one that takes several list entries a turn where a
-// list can be that long, unless four poses share a warp (mixed precision, small ligands).
-void* split_fwd(const SplitKernels& kn, int cap, int warps, int precision, bool small) {
-  return cap >= 2 * kLongTurns * warps && !(precision == BD_PREC_MIXED && small) ? kn.fwd_long : kn.fwd;
+// The ligand-atom kernel of a pool of `cap` slots: four poses a warp for small ligands in mixed precision,
+// several list entries a turn, each where a list can be that long, else one.
+void* split_fwd(const SplitKernels& kn, int cap, int warps, bool small) {
+  return small && kn.fwd_packed && cap > 4 * warps ? kn.fwd_packed : cap >= 2 * kLongTurns * warps ? kn.fwd_long : kn.fwd;
 }
 
 int enqueue_split_launch(BdHandle* h, int K, cudaStream_t s, int cur, bool capture) {
@@ -1551,7 +1551,7 @@ int enqueue_split_launch(BdHandle* h, int K, cudaStream_t s, int cur, bool captu
   stepper_smem(h->S, h->P, kn.last);
   p.b_step = persistent_blocks(h, kn.mid, kStepBlock, p.smem);
   p.b_fwd = persistent_blocks(h, kn.fwd, 256);
-  p.fwd = split_fwd(kn, h->buf[0].cap, 8 * p.b_fwd, h->sp.precision, h->S.n_lig <= 32 && !h->S.wca);
+  p.fwd = split_fwd(kn, h->buf[0].cap, 8 * p.b_fwd, h->S.n_lig <= 32 && !h->S.wca);
   p.b_rev = persistent_blocks(h, kn.rev, 256);
   p.side = capture ? h->side : nullptr;
   p.fork = h->fork;
@@ -2027,7 +2027,7 @@ int enqueue_multi_launch(BdMulti* m, int K, cudaStream_t s, int c, bool capture)
   SplitPlan p{&kn, kn.fwd, &T, m->split, m->rev, 0};
   p.b_step = blocks(kn.mid, kStepBlock);
   p.b_fwd = blocks(kn.fwd, 256);
-  p.fwd = split_fwd(kn, m->cap, 8 * p.b_fwd, m->precision, m->T.small);
+  p.fwd = split_fwd(kn, m->cap, 8 * p.b_fwd, m->T.small);
   p.b_rev = blocks(kn.rev, 256);
   p.side = capture ? m->side : nullptr;
   p.fork = m->fork;

@@ -27,7 +27,6 @@ struct MultiTab {
   __device__ __forceinline__ const DevSim& sim(int k) const { return sim_[k]; }
   __device__ __forceinline__ int locate(int& id) const;
   __device__ __forceinline__ int global_id(int k, int id) const { return (int)(base[k] + id); }
-  __device__ __forceinline__ bool small_ligands() const { return small; }
   __device__ __forceinline__ bool large_ligands() const { return large; }
   __device__ __forceinline__ int largest_ligand() const { return largest; }
   __device__ __forceinline__ void refill(Traj& tr, int& k, bool& dead, int lane) const;

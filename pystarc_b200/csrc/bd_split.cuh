@@ -66,8 +66,6 @@ struct OneTab {
   __device__ __forceinline__ const DevSim& sim(int) const { return P; }
   __device__ __forceinline__ int locate(int&) const { return 0; }  // trajectory id -> system, local id
   __device__ __forceinline__ int global_id(int, int id) const { return id; }
-  // every ligand has at most 32 atoms and no contact forces (which a whole warp evaluates)
-  __device__ __forceinline__ bool small_ligands() const { return S.n_lig <= 32 && !S.wca; }
   // ligands worth sharing among warps: every one of at least 128 atoms, no contact forces
   __device__ __forceinline__ bool large_ligands() const { return S.n_lig >= 128 && !S.wca; }
   __device__ __forceinline__ int largest_ligand() const { return S.n_lig; }  // atoms
@@ -395,7 +393,7 @@ __device__ __forceinline__ int fwd_warps(int n, int n_warps) {
   return n <= n_warps / 8 ? 8 : n <= n_warps / 4 ? 4 : n <= n_warps / 2 ? 2 : 1;
 }
 
-// List entries a warp takes at a time in split_fwd_kernel<LONG>: about eight turns per warp and at most 16
+// List entries a warp takes at a time in split_fwd_kernel<FWD_LONG>: about eight turns per warp and at most 16
 // entries, or 512 atoms of ligands above 64 (a last turn of long poses would leave other warps waiting).
 // The cursor is one address, and the device adds to it about once a nanosecond: with an entry a turn, lists
 // of 100,000 poses and more were bound by it (256 steps, far-field of 18 atoms, FP64: 300,000 poses
@@ -412,9 +410,12 @@ __device__ __forceinline__ int fwd_turn(int n, int n_warps, int atoms) {
 // ligands in mixed precision and lists of several poses a warp (18 atoms, 150,000 slots: 155 -> 116 us;
 // at 8,000 slots a warp per pose is the faster, 15.5 against 17.4 us, and in FP64 the quarter-warp
 // form spills and is slower at 30,011).  Bound by latency at 13 warps per SM: issue slots 45 %, L1 43 %,
-// the double-float conversions 22 %.  LONG: several entries a turn, for pools that can list 16 poses per
-// warp; a kernel of its own, because the loop over a turn cost lists with one entry a turn 2 %.
-template <typename FT, bool TORQUE, bool LONG, class TAB>
+// the double-float conversions 22 %.  FORM: a kernel each for one list entry a turn, for several (pools that
+// can list 16 poses per warp) and for four poses a warp (small ligands in mixed precision, which fall back to
+// one a turn on short lists): the loop over a turn costs lists with one entry a turn 2 %, the code of the
+// four poses 1 to 5 % (40 atoms, mixed with torque, 20,000 slots, 256 steps: 9.42 -> 9.03 ms).
+enum { FWD_ONE, FWD_LONG, FWD_PACKED };
+template <typename FT, bool TORQUE, int FORM, class TAB>
 __global__ void __launch_bounds__(256, 2) split_fwd_kernel(const __grid_constant__ TAB T, SlotBuf B, SplitBuf U,
                                                            int set) {
   const unsigned FULL = 0xffffffffu;
@@ -425,7 +426,7 @@ __global__ void __launch_bounds__(256, 2) split_fwd_kernel(const __grid_constant
   // Entries of the list that go four to a warp.  With torque the one to three after them take a warp each, one
   // that has few of the others; without, the lanes past the end repeat a pose, uncounted (with the counts apart
   // the torque kernel spills 40 bytes more: 150,000 slots +1 %; the tail in the loop below costs the other 1 %).
-  const int packed = sizeof(FT) == 4 && !LONG && T.small_ligands() && n > 4 * n_warps ? (TORQUE ? n & ~3 : n) : 0;
+  const int packed = FORM == FWD_PACKED && n > 4 * n_warps ? (TORQUE ? n & ~3 : n) : 0;
   if (packed) {
     // lanes read the poses of `m` list entries together, then hand them out four at a time
     const int m = min(32, 4 * ((packed + 4 * n_warps - 1) / (4 * n_warps)));
@@ -481,7 +482,7 @@ __global__ void __launch_bounds__(256, 2) split_fwd_kernel(const __grid_constant
       }
     }
   } else {
-    const int m = LONG ? fwd_turn(n, n_warps, T.largest_ligand()) : 1;
+    const int m = FORM == FWD_LONG ? fwd_turn(n, n_warps, T.largest_ligand()) : 1;
     for (int j = TORQUE && packed ? packed + n_warps - 1 - first : first * m, left = m; j < n;) {
       const int slot = U.flist[j];
       int id = B.traj[slot];
@@ -492,7 +493,7 @@ __global__ void __launch_bounds__(256, 2) split_fwd_kernel(const __grid_constant
                                                              PosFromPose{pose.R, pose.c}, f, t, e, cnt,
                                                              RecView{nullptr, nullptr});
       store_force(U, slot, lane, f, t);
-      if (LONG && --left) ++j;
+      if (FORM == FWD_LONG && --left) ++j;
       else if (TORQUE && packed) break;
       else {
         j = m * next_item(U.cnt + 4 * set + 2, n_warps, lane);

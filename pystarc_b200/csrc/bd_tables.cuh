@@ -15,7 +15,7 @@ constexpr int kGroups[5] = {1, 4, 8, 16, 32};  // lanes per trajectory of step_k
 
 struct SplitKernels {
   void *first, *mid, *last;  // scalar kernel: begin, end + begin, end
-  void *fwd, *fwd_long, *rev;
+  void *fwd, *fwd_long, *fwd_packed, *rev;  // packed: null in FP64
 };
 
 struct KernelTable {
@@ -28,9 +28,11 @@ struct KernelTable {
 
 template <typename FT, bool TQ, class TAB>
 SplitKernels split_kernels() {
+  void* packed = nullptr;
+  if constexpr (sizeof(FT) == 4) packed = (void*)&split_fwd_kernel<FT, TQ, FWD_PACKED, TAB>;
   return {(void*)&split_step_kernel<FT, TQ, false, true, TAB>, (void*)&split_step_kernel<FT, TQ, true, true, TAB>,
-          (void*)&split_step_kernel<FT, TQ, true, false, TAB>, (void*)&split_fwd_kernel<FT, TQ, false, TAB>,
-          (void*)&split_fwd_kernel<FT, TQ, true, TAB>, (void*)&split_rev_kernel<FT, TQ, TAB>};
+          (void*)&split_step_kernel<FT, TQ, true, false, TAB>, (void*)&split_fwd_kernel<FT, TQ, FWD_ONE, TAB>,
+          (void*)&split_fwd_kernel<FT, TQ, FWD_LONG, TAB>, packed, (void*)&split_rev_kernel<FT, TQ, TAB>};
 }
 
 template <typename FT, bool TQ>
